@@ -92,7 +92,7 @@ typedef struct ngrav_gpu_diag {
     double com[3];         /* centre of mass */
     double L[3];           /* angular momentum about the COM */
     double P[3];           /* linear momentum */
-    int potential_exact;   /* 1: exact pairwise sum in FP64; 2: exact pair set, FP32 pair terms; 0: none (NaN) */
+    int potential_exact;   /* 1: exact pairwise sum to FP64 accuracy; 2: exact pair set, FP32 pair terms; 0: none (NaN) */
 } ngrav_gpu_diag;
 
 typedef struct ngrav_gpu_ferr {
@@ -237,11 +237,13 @@ int ngrav_gpu_get_state(ngrav_gpu_ctx* ctx, double* x, double* y, double* z, dou
 int ngrav_gpu_get_accel(ngrav_gpu_ctx* ctx, double* ax, double* ay, double* az);
 
 /* FP64 conservation diagnostics of the current state.  exact_potential:
- * 1 = exact O(N^2) pairwise potential on the GPU, every pair term in FP64;
+ * 1 = exact O(N^2) pairwise potential on the GPU, every pair term to FP64
+ *     accuracy (in FP64 below 4,096 particles, as a pair of floats above,
+ *     with FP64 sums; the sum's error is that of FP64 terms);
  * 2 = the same pair set with FP32 pair terms and FP64 sums (the offset of a
  *     pair formed from the double-float positions, so its error is of order
  *     2^-24 of the separation; Plummer softening, a spline run takes mode 1),
- *     about 2.5 s at n = 4,194,304 where mode 1 takes minutes;
+ *     about 2.5 s at n = 4,194,304 where mode 1 takes tens of seconds;
  * 0 = mode 1 up to 262,144 particles, else no potential (NaN).
  * out->potential_exact reports the mode used (0, 1 or 2). */
 int ngrav_gpu_diagnostics(ngrav_gpu_ctx* ctx, int exact_potential, ngrav_gpu_diag* out);

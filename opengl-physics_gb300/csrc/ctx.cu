@@ -955,13 +955,22 @@ int ngrav_gpu_diagnostics(ngrav_gpu_ctx* ctx, int exact_potential, ngrav_gpu_dia
         for (int b = 0; b < pb; ++b) pot += hp[b];
         out->potential = ctx->opts.G * pot;
     } else if (exact) {
-        launch_potential(n, ctx->P, split, ctx->opts.eps * ctx->opts.eps, spline_h(ctx), ctx->dpartial, ctx->stream);
+        const double mscale =
+            potential_scaled(n) && std::isfinite(M) && M != 0.0 ? std::ldexp(1.0, -std::ilogb(M)) : 1.0;
+        launch_potential(n, ctx->P, split, ctx->opts.eps * ctx->opts.eps, spline_h(ctx), mscale, ctx->dpartial,
+                         ctx->stream);
         NG_CUDA(cudaMemcpyAsync(h.data(), ctx->dpartial, sizeof(double) * npb, cudaMemcpyDeviceToHost,
                                 ctx->stream));
         NG_CUDA(cudaStreamSynchronize(ctx->stream));
-        double pot = 0.0;
-        for (int b = 0; b < npb; ++b) pot += h[b];
-        out->potential = ctx->opts.G * pot;
+        // Neumaier's compensated sum: thousands of block partials of one sign
+        double pot = 0.0, low = 0.0;
+        for (int b = 0; b < npb; ++b) {
+            const double t = pot + h[b];
+            low += std::abs(pot) >= std::abs(h[b]) ? (pot - t) + h[b] : (h[b] - t) + pot;
+            pot = t;
+        }
+        if (std::isfinite(low)) pot += low;
+        out->potential = ctx->opts.G * (pot / mscale / mscale);
     } else {
         out->potential = std::nan("");
     }

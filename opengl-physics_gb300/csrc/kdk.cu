@@ -11,8 +11,7 @@
 // Diagnostics (restating include/ngrav/System.hpp:119-193 and
 // src/DeckSim.cpp:147-153): kinetic energy, centre of mass, angular momentum
 // about the COM and linear momentum are FP64 block reductions combined in a
-// fixed order (deterministic); the potential is the exact FP64 pair sum
-// sum_{i<j} -G m_i m_j / sqrt(r^2 + eps^2).
+// fixed order (deterministic); the exact pair potential is potential.cu's.
 #include "engine.cuh"
 
 #include <algorithm>
@@ -397,74 +396,7 @@ void launch_diag_pass2(long long n, const Particles& P, bool split, double cx, d
                                                               partial);
 }
 
-// Exact pair potential: thread i sums j > i over shared-memory tiles, in FP64.
-constexpr int kPotThreads = 256;
-
-// spline_h > 0: the spline pair potential of smoothing length spline_h
-// (softening.cuh); else Plummer with eps2.
-__global__ void __launch_bounds__(kPotThreads) potential_kernel(long long n, const float4* __restrict__ pos,
-                                                                const float4* __restrict__ plo, double eps2,
-                                                                double spline_h, double* __restrict__ partial) {
-    __shared__ double sx[kPotThreads], sy[kPotThreads], sz[kPotThreads], sm[kPotThreads];
-    __shared__ double red[32];
-    const long long i = blockIdx.x * (long long)kPotThreads + threadIdx.x;
-    double xi = 0, yi = 0, zi = 0, mi = 0;
-    if (i < n) {
-        const float4 p = pos[i];
-        xi = p.x;
-        yi = p.y;
-        zi = p.z;
-        mi = p.w;
-        if (plo) {
-            const float4 l = plo[i];
-            xi += (double)l.x;
-            yi += (double)l.y;
-            zi += (double)l.z;
-        }
-    }
-    double local = 0.0;
-    const long long first_tile = blockIdx.x * (long long)kPotThreads;
-    for (long long t = first_tile; t < n; t += kPotThreads) {
-        const long long j = t + threadIdx.x;
-        __syncthreads();
-        if (j < n) {
-            const float4 p = pos[j];
-            double x = p.x, y = p.y, z = p.z;
-            if (plo) {
-                const float4 l = plo[j];
-                x += (double)l.x;
-                y += (double)l.y;
-                z += (double)l.z;
-            }
-            sx[threadIdx.x] = x;
-            sy[threadIdx.x] = y;
-            sz[threadIdx.x] = z;
-            sm[threadIdx.x] = p.w;
-        }
-        __syncthreads();
-        if (i < n) {
-            const int kmax = (int)min((long long)kPotThreads, n - t);
-            for (int k = 0; k < kmax; ++k) {
-                if (t + k <= i) continue;
-                const double dx = sx[k] - xi, dy = sy[k] - yi, dz = sz[k] - zi;
-                if (spline_h > 0.0) {
-                    const double r = sqrt(dx * dx + dy * dy + dz * dz);
-                    local += sm[k] * spline_phi_d(r / spline_h) / spline_h;
-                } else {
-                    const double r2 = dx * dx + dy * dy + dz * dz + eps2;
-                    local -= sm[k] * rsqrt(r2);
-                }
-            }
-        }
-    }
-    local *= mi;
-    const double t = block_sum_d(local, red);
-    if (threadIdx.x == 0) partial[blockIdx.x] = t;
-}
-
-int potential_blocks(long long n) { return (int)((n + kPotThreads - 1) / kPotThreads); }
-
-// The same pair set (every i < j, Plummer) with FP32 pair terms and FP64
+// Pair potential over every i < j (Plummer) with FP32 pair terms and FP64
 // sums, for sizes where the FP64 pipe is too slow (n = 4M: 8.8e12 pairs).
 // Thread = target i; sources staged through shared memory as double-float
 // positions, each offset formed as (hi_j - hi_i) + (lo_j - lo_i) in FP32 (an
@@ -531,12 +463,6 @@ int potential_f32_blocks(long long n, int sm_count) {
 void launch_potential_f32(long long n, const Particles& P, bool split, double eps2, int blocks, double* partial,
                           cudaStream_t s) {
     potential_f32_kernel<<<blocks, kPot32Threads, 0, s>>>(n, P.pos, split ? P.plo : nullptr, (float)eps2, partial);
-}
-
-void launch_potential(long long n, const Particles& P, bool split, double eps2, double spline_h, double* partial,
-                      cudaStream_t s) {
-    potential_kernel<<<potential_blocks(n), kPotThreads, 0, s>>>(n, P.pos, split ? P.plo : nullptr, eps2, spline_h,
-                                                                 partial);
 }
 
 // ---------------------------------------------------------------------------

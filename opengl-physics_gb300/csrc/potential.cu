@@ -1,0 +1,459 @@
+// potential.cu -- the exact pair potential of the conservation diagnostics,
+// sum over i < j of -m_i m_j / sqrt(r^2 + eps^2) (Plummer) or m_i m_j phi(r/h)/h
+// (spline), restating System::TotalEnergy (include/ngrav/System.hpp:119-150).
+//
+// Every pair term is needed to double-precision accuracy, and GB300's FP64
+// pipe runs at 1/64 of the FP32 rate: an FP64 pair costs about 21 FP64
+// operations, 1,344 FP32 slots.  potential_df_kernel forms each term on the
+// packed FP32 pipe as an unevaluated pair of floats instead, in about 52 FP32
+// operations, and leaves FP64 to the sums (one flush per 32 sources):
+//
+//  * Frame.  Targets and sources of a (128 targets, 32 sources) tile are taken
+//    relative to the tile's middle target and scaled by a power of two so the
+//    largest |coordinate| E lies in [1/2, 1).  Each coordinate is split into
+//    x1 on the grid 2^-22 and the rest x2, so a difference of two x1 is exact
+//    in one subtraction and the difference of two x2 is off by 2^-48 E only.
+//  * r^2 + eps^2.  B = the FP32 sum of squares seeds three fused steps h += s^2
+//    that all round at B's exponent; h_k - h_(k-1) is then exact (Sterbenz) and
+//    one more fma recovers what each step rounded off, so B plus the collected
+//    remainder is r^2 + eps^2 to about 2^-46.
+//  * 1/r.  The hardware reciprocal square root y0 of B, with the residual
+//    e = 1 - (r^2 + eps^2) y0^2 taken by fma: y = y0 (1 + e/2 + 3/8 e^2).
+//  * Sum.  m y0 + m corr as a float pair, two-sum accumulated over 32 sources,
+//    then added to the thread's FP64 total.
+//
+// The x2 differences limit close pairs (E / r x 2^-47), so a pair nearer than
+// E/16 is formed again from the particles' own double-float positions with
+// error-free differences (refine_pair), and pairs inside the spline's kernel,
+// at r = 0 or outside FP32's range take the FP64 formula.  Emulated on the
+// CPU with exact rounding against 80-bit sums (Plummer spheres, eps 0 to
+// 0.05): the sum's relative error at n >= 4,096 is 1e-16 to 5e-16, the same
+// as with FP64 terms (1e-16 to 8e-16); at n = 1,000 it is 1e-15 against 1e-16
+// (too few terms to average over), hence kPotDfMin.
+//
+// Measured (GB300, one diagnostics call on a Plummer sphere in tree order):
+// 131,071 particles 299 ms with FP64 terms -> 17.1 ms (0.70 of the FP32 pipe's
+// 52-operation time), 16,384 15.0 -> 0.35 ms, 2,048 (FP64 blocks of 32 sources
+// instead of whole rows) 1.87 -> 0.17 ms; spline, 20,011: 53.6 -> 0.66 ms.
+// Particles not yet in tree order have wide frames, so more pairs take
+// refine_pair: 45 ms at 131,071.
+#include "ctx_kernels.cuh"
+#include "engine.cuh"
+#include "softening.cuh"
+
+#include <algorithm>
+
+namespace ngrav {
+
+constexpr int kPotThreads = 128;           // targets per block
+constexpr int kPotSub = 32;                // sources per frame (one staging warp)
+constexpr int kPotChunkMax = 8192;         // sources per block at most, but no more than
+constexpr int kPotChunks = 16;             //   this many blocks per target tile
+// Smallest n of the double-float kernel.  Below it FP64 terms are exact to
+// the last bit of the sum and cheap (4,095: 8.4 M pairs).
+constexpr long long kPotDfMin = 4096;
+constexpr float kPotNear2 = 1.f / 512.f;   // (E/16)^2 at E = 1/sqrt(2); E is in [1/2, 1)
+
+// Sources per block: whole frames, few enough that the triangle's blocks
+// fill the GPU several times over (152 SMs x 4 CTAs x 6), up to kPotChunkMax
+// or a kPotChunks-th of n.
+static long long potential_chunk(long long n) {
+    const long long unit = n < kPotDfMin ? kPotSub : kPotThreads;
+    const long long want = n * n / (2LL * kPotThreads * 152 * 4 * 6);  // n < 2^31: no overflow
+    const long long most = std::max<long long>(kPotChunkMax, (n + kPotChunks - 1) / kPotChunks);
+    return (std::min(most, std::max(unit, want)) + unit - 1) / unit * unit;
+}
+
+static long long pot_tiles(long long n) { return (n + kPotThreads - 1) / kPotThreads; }
+static long long pot_chunks(long long n) { return (n + potential_chunk(n) - 1) / potential_chunk(n); }
+
+int potential_blocks(long long n) { return (int)std::max<long long>(1, pot_tiles(n) * pot_chunks(n)); }
+
+// ---------------------------------------------------------------------------
+// FP32 and packed FP32 steps under one name (no step may be contracted or
+// reassociated: the error-free transformations depend on each rounding).
+// ---------------------------------------------------------------------------
+
+// A packed operand has no free negation, so differences are fused steps with
+// -1 (the same rounding) and signs are carried where they are needed.
+__device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float vsub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float vrsqrt(float a) { return rsqrtf(a); }
+__device__ __forceinline__ float vneg(float a) { return -a; }
+__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 vsub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+__device__ __forceinline__ float2 vrsqrt(float2 a) { return make_float2(rsqrtf(a.x), rsqrtf(a.y)); }
+__device__ __forceinline__ float2 vneg(float2 a) { return make_float2(-a.x, -a.y); }
+template <class V>
+__device__ __forceinline__ V splat(float v);
+template <>
+__device__ __forceinline__ float splat<float>(float v) { return v; }
+template <>
+__device__ __forceinline__ float2 splat<float2>(float v) { return make_float2(v, v); }
+
+// a + b = s + e exactly.
+template <class V>
+__device__ __forceinline__ void sum2(V a, V b, V& s, V& e) {
+    s = vadd(a, b);
+    const V bb = vsub(s, a);
+    e = vadd(vsub(a, vsub(s, bb)), vsub(b, bb));
+}
+
+// What one fused step h += s^2 rounded off, plus l (2 s + l): the axis's
+// share of r^2 that the running sum does not hold.  `h` moves on.
+template <class V>
+__device__ __forceinline__ V square_step(V s, V l, V& h) {
+    const V h2 = vfma(s, s, h);
+    const V nd = vsub(h, h2);
+    const V f = vfma(vfma(splat<V>(2.f), s, l), l, vfma(s, s, nd));
+    h = h2;
+    return f;
+}
+
+// B: FP32 r^2 + eps^2 from the leading differences.
+template <class V>
+__device__ __forceinline__ V lead_r2(const V s[3], V e2h) {
+    return vfma(s[0], s[0], vfma(s[1], s[1], vfma(s[2], s[2], e2h)));
+}
+
+// 1 / sqrt(|s + l|^2 + eps^2) as y0 + corr, B = lead_r2(s); ny0 = -y0.
+template <class V>
+__device__ __forceinline__ void inv_dist(const V s[3], const V l[3], V e2h, V e2l, V B, V& y0, V& ny0, V& corr) {
+    y0 = vrsqrt(B);
+    ny0 = vneg(y0);
+    V h = B;
+    const V f0 = square_step(s[0], l[0], h);
+    const V f1 = square_step(s[1], l[1], h);
+    const V f2 = square_step(s[2], l[2], h);
+    const V h4 = vadd(h, e2h);
+    const V f3 = vadd(vadd(e2h, vsub(h, h4)), e2l);
+    const V rest = vadd(vadd(f0, f1), vadd(f2, f3));
+    const V low = vadd(vfma(splat<V>(-2.f), B, h4), rest);  // r^2 + eps^2 - B
+    const V nz = vmul(B, ny0);
+    const V v = vfma(low, y0, vfma(B, y0, nz));
+    const V e = vfma(v, ny0, vfma(nz, y0, splat<V>(1.f)));
+    corr = vmul(y0, vmul(e, vfma(splat<V>(0.375f), e, splat<V>(0.5f))));
+}
+
+// ---------------------------------------------------------------------------
+// Pairs the frame cannot resolve
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ double pair_phi(double dx, double dy, double dz, double eps2, double spline_h) {
+    // -potential of a unit-mass pair
+    if (spline_h > 0.0) {
+        const double r = sqrt(dx * dx + dy * dy + dz * dz);
+        return -spline_phi_d(r / spline_h) / spline_h;
+    }
+    return rsqrt(dx * dx + dy * dy + dz * dz + eps2);
+}
+
+struct PotPair {
+    float y, corr;  // double-float 1/r in the frame's unit (0, 0 when `wide` holds the term)
+    double wide;    // 1/r or the spline's -phi/h in FP64, in the caller's unit
+};
+
+// One pair from the double-float positions themselves: difference of the
+// high halves and of the low halves error-free, merged into a normalised
+// float pair per axis.
+__device__ __noinline__ PotPair refine_pair(float4 th, float4 tl, float4 qh, float4 ql, float sc, float e2h,
+                                            float e2l, float kernel2, double eps2, double spline_h) {
+    const float a[3] = {qh.x, qh.y, qh.z}, al[3] = {ql.x, ql.y, ql.z};
+    const float b[3] = {th.x, th.y, th.z}, bl[3] = {tl.x, tl.y, tl.z};
+    float s[3], l[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        float d, de, q, qe, u, ue;
+        sum2(a[k], -b[k], d, de);
+        sum2(al[k], -bl[k], q, qe);
+        sum2(de, q, u, ue);
+        float hi, lo;
+        sum2(d, u, hi, lo);
+        s[k] = hi * sc;
+        l[k] = (lo + (qe + ue)) * sc;
+    }
+    const float B = lead_r2(s, e2h);
+    PotPair r = {0.f, 0.f, 0.0};
+    // FP32 resolves the pair: neither inside the spline's kernel nor near the
+    // ends of its range (a NaN fails both)
+    if (B >= kernel2 && B >= 1e-20f && B <= 16.f) {
+        float ny;
+        inv_dist(s, l, e2h, e2l, B, r.y, ny, r.corr);
+        return r;
+    }
+    const double dx = ((double)qh.x + (double)ql.x) - ((double)th.x + (double)tl.x);
+    const double dy = ((double)qh.y + (double)ql.y) - ((double)th.y + (double)tl.y);
+    const double dz = ((double)qh.z + (double)ql.z) - ((double)th.z + (double)tl.z);
+    r.wide = pair_phi(dx, dy, dz, eps2, spline_h);
+    return r;
+}
+
+// ---------------------------------------------------------------------------
+// Double-float kernel
+// ---------------------------------------------------------------------------
+
+struct __align__(16) PotStage {
+    float x1[3][kPotThreads];  // source coordinates in the frame: grid part
+    float x2[3][kPotThreads];  //   and the rest
+    float m[kPotThreads];      // mass x mscale x frame scale
+    float sc[kPotThreads / kPotSub], e2h[kPotThreads / kPotSub], e2l[kPotThreads / kPotSub],
+        near2[kPotThreads / kPotSub], kernel2[kPotThreads / kPotSub];
+};
+
+// x - c for a double-float x, as a normalised float pair.
+__device__ __forceinline__ void rel_coord(float xh, float xl, float c, float& yh, float& yl) {
+    float d, e;
+    sum2(xh, -c, d, e);
+    const float u = e + xl;
+    yh = d + u;
+    yl = u - (yh - d);
+}
+
+// y scaled by sc, split at the grid 2^-22 (|y sc| < 1).
+__device__ __forceinline__ void grid_split(float yh, float yl, float sc, float& x1, float& x2) {
+    x1 = __fadd_rn(__fmaf_rn(yh, sc, 3.f), -3.f);
+    x2 = __fmaf_rn(yl, sc, __fmaf_rn(yh, sc, -x1));
+}
+
+// Double total of a block (thread 0).
+__device__ __forceinline__ double pot_block_sum(double v) {
+    __shared__ double sh[kPotThreads / 32];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double t = 0.0;
+    for (int k = 0; k < kPotThreads / 32; ++k) t += sh[k];
+    return t;
+}
+
+// Block (I, c): targets of tile I against sources [128 I + c chunk, + chunk),
+// pairs i < j.  FP32-pipe bound: 52 operations per pair, two sources per
+// packed instruction.  partial[c gridDim.x + I] (0 past the end).
+template <bool SPLIT>
+__global__ void __launch_bounds__(kPotThreads, 5) potential_df_kernel(long long n, const float4* __restrict__ pos,
+                                                                      const float4* __restrict__ plo, double eps2,
+                                                                      double spline_h, double mscale, long long chunk,
+                                                                      double* __restrict__ partial) {
+    __shared__ PotStage sm;
+    __shared__ unsigned s_rho;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const long long i0 = blockIdx.x * (long long)kPotThreads;
+    const long long j_begin = i0 + blockIdx.y * chunk;
+    double* out = partial + (blockIdx.y * (long long)gridDim.x + blockIdx.x);
+    if (j_begin >= n) {
+        if (tid == 0) *out = 0.0;
+        return;
+    }
+    const long long j_end = j_begin + chunk < n ? j_begin + chunk : n;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const long long i = i0 + tid;
+    const bool have = i < n;
+    const float4 th = have ? pos[i] : zero;
+    const float4 tl = (SPLIT && have) ? plo[i] : zero;
+    const float4 c = pos[i0 + kPotThreads / 2 < n ? i0 + kPotThreads / 2 : n - 1];
+    float th_[3] = {0.f, 0.f, 0.f}, tl_[3] = {0.f, 0.f, 0.f};
+    if (have) {
+        rel_coord(th.x, tl.x, c.x, th_[0], tl_[0]);
+        rel_coord(th.y, tl.y, c.y, th_[1], tl_[1]);
+        rel_coord(th.z, tl.z, c.z, th_[2], tl_[2]);
+    }
+    if (tid == 0) s_rho = __float_as_uint(fmaxf(1e-30f, (float)sqrt(spline_h > 0.0 ? 0.0 : eps2)));
+    __syncthreads();
+    {  // largest target coordinate (float bits of |y| order like the value; a NaN sorts above)
+        const unsigned a = max(max(__float_as_uint(fabsf(th_[0])), __float_as_uint(fabsf(th_[1]))),
+                               __float_as_uint(fabsf(th_[2])));
+        const unsigned r = __reduce_max_sync(0xffffffffu, a);
+        if (lane == 0) atomicMax(&s_rho, r);
+    }
+    double acc = 0.0;
+    for (long long t = j_begin; t < j_end; t += kPotThreads) {
+        __syncthreads();
+        {  // stage: warp w fills frame w
+            const long long j = t + tid;
+            const bool in = j < j_end;
+            const float4 q = in ? pos[j] : zero;
+            const float4 ql = (SPLIT && in) ? plo[j] : zero;
+            float yh[3] = {0.f, 0.f, 0.f}, yl[3] = {0.f, 0.f, 0.f};
+            if (in) {
+                rel_coord(q.x, ql.x, c.x, yh[0], yl[0]);
+                rel_coord(q.y, ql.y, c.y, yh[1], yl[1]);
+                rel_coord(q.z, ql.z, c.z, yh[2], yl[2]);
+            }
+            unsigned a = max(max(__float_as_uint(fabsf(yh[0])), __float_as_uint(fabsf(yh[1]))),
+                             __float_as_uint(fabsf(yh[2])));
+            a = max(__reduce_max_sync(0xffffffffu, a), s_rho);
+            // 2^-ex with E = 2^ex [1/2, 1); an E outside FP32's comfortable
+            // range (or a NaN) sends every pair of the frame to refine_pair,
+            // and from there to FP64
+            const unsigned eb = a >> 23;
+            const bool fits = eb >= 8u && eb <= 245u;
+            const float sc = fits ? __uint_as_float((253u - eb) << 23) : 1.f;
+            const double scd = (double)sc, e2 = spline_h > 0.0 || !fits ? 0.0 : eps2 * scd * scd;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                float x1, x2;
+                grid_split(yh[k], yl[k], sc, x1, x2);
+                sm.x1[k][tid] = fits ? x1 : 0.f;
+                sm.x2[k][tid] = fits ? x2 : 0.f;
+            }
+            sm.m[tid] = (float)((double)q.w * mscale * scd);
+            if (lane == 0) {
+                const float inf = __uint_as_float(0x7f800000u);
+                // rounded up, so that every pair inside the kernel is caught
+                const float k2 = spline_h > 0.0 ? (float)(4.00001 * (spline_h * scd) * (spline_h * scd)) : 0.f;
+                sm.sc[w] = sc;
+                sm.e2h[w] = (float)e2;
+                sm.e2l[w] = (float)(e2 - (double)(float)e2);
+                sm.kernel2[w] = fits ? k2 : inf;
+                sm.near2[w] = fits ? fmaxf(kPotNear2, k2) : inf;
+            }
+        }
+        __syncthreads();
+        const int frames = (int)((min((long long)kPotThreads, j_end - t) + kPotSub - 1) / kPotSub);
+        for (int f = 0; f < frames; ++f) {
+            const float sc = sm.sc[f], near2 = sm.near2[f];
+            const float2 e2h = splat<float2>(sm.e2h[f]), e2l = splat<float2>(sm.e2l[f]);
+            float2 n1[3], n2[3];  // the target, negated
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                float x1, x2;
+                grid_split(th_[k], tl_[k], sc, x1, x2);
+                n1[k] = splat<float2>(-x1);
+                n2[k] = splat<float2>(-x2);
+            }
+            const long long jf = t + f * kPotSub;
+            const bool diag = jf < i0 + kPotThreads;  // sources at or before some target
+            float2 A = make_float2(0.f, 0.f), R = A;
+            for (int k4 = 0; k4 < kPotSub; k4 += 4) {
+                float4 q1[3], q2[3];
+#pragma unroll
+                for (int x = 0; x < 3; ++x) {
+                    q1[x] = *reinterpret_cast<const float4*>(&sm.x1[x][f * kPotSub + k4]);
+                    q2[x] = *reinterpret_cast<const float4*>(&sm.x2[x][f * kPotSub + k4]);
+                }
+                const float4 qm = *reinterpret_cast<const float4*>(&sm.m[f * kPotSub + k4]);
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const long long j0 = jf + k4 + 2 * half;
+                    float2 s[3], l[3], m = half ? make_float2(qm.z, qm.w) : make_float2(qm.x, qm.y);
+#pragma unroll
+                    for (int x = 0; x < 3; ++x) {
+                        s[x] = vadd(half ? make_float2(q1[x].z, q1[x].w) : make_float2(q1[x].x, q1[x].y), n1[x]);
+                        l[x] = vadd(half ? make_float2(q2[x].z, q2[x].w) : make_float2(q2[x].x, q2[x].y), n2[x]);
+                    }
+                    if (diag) {
+                        if (j0 <= i) m.x = 0.f;
+                        if (j0 + 1 <= i) m.y = 0.f;
+                    }
+                    const float2 B = lead_r2(s, e2h);
+                    float2 y0, ny0, corr;
+                    inv_dist(s, l, e2h, e2l, B, y0, ny0, corr);
+                    if (!(fminf(B.x, B.y) >= near2)) {
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            if ((u ? B.y : B.x) >= near2) continue;
+                            const long long j = j0 + u;
+                            float y = 0.f, co = 0.f;
+                            if (have && j > i && j < j_end) {
+                                const float4 qh = pos[j];
+                                const PotPair p = refine_pair(th, tl, qh, SPLIT ? plo[j] : zero, sc, e2h.x, e2l.x,
+                                                              sm.kernel2[f], eps2, spline_h);
+                                y = p.y;
+                                co = p.corr;
+                                acc += (double)qh.w * mscale * p.wide;
+                            }
+                            if (u) {
+                                y0.y = y;
+                                ny0.y = -y;
+                                corr.y = co;
+                            } else {
+                                y0.x = y;
+                                ny0.x = -y;
+                                corr.x = co;
+                            }
+                        }
+                    }
+                    const float2 ph = vmul(m, y0);
+                    const float2 npe = vfma(m, ny0, ph);  // what ph rounded off m y0, negated
+                    float2 S, er;
+                    sum2(A, ph, S, er);
+                    A = S;
+                    R = vadd(R, vsub(vfma(m, corr, er), npe));
+                }
+            }
+            float S, er;
+            sum2(A.x, A.y, S, er);
+            acc += (double)S;
+            acc += (double)(er + (R.x + R.y));
+        }
+    }
+    const double t = pot_block_sum(have ? -(double)th.w * mscale * acc : 0.0);
+    if (tid == 0) *out = t;
+}
+
+// ---------------------------------------------------------------------------
+// FP64 kernel (small n): the same blocks, FP64-pipe bound, so the triangle is
+// cut into blocks of 32 sources to spread over the SMs.
+// ---------------------------------------------------------------------------
+
+__global__ void __launch_bounds__(kPotThreads) potential_f64_kernel(long long n, const float4* __restrict__ pos,
+                                                                    const float4* __restrict__ plo, double eps2,
+                                                                    double spline_h, long long chunk,
+                                                                    double* __restrict__ partial) {
+    __shared__ double sx[kPotSub], sy[kPotSub], sz[kPotSub], smm[kPotSub];
+    const int tid = threadIdx.x;
+    const long long i0 = blockIdx.x * (long long)kPotThreads;
+    const long long j_begin = i0 + blockIdx.y * chunk;
+    double* out = partial + (blockIdx.y * (long long)gridDim.x + blockIdx.x);
+    if (j_begin >= n) {
+        if (tid == 0) *out = 0.0;
+        return;
+    }
+    const long long j_end = j_begin + chunk < n ? j_begin + chunk : n;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const long long i = i0 + tid;
+    const float4 p = i < n ? pos[i] : zero;
+    const float4 l = (plo && i < n) ? plo[i] : zero;
+    const double xi = (double)p.x + (double)l.x, yi = (double)p.y + (double)l.y, zi = (double)p.z + (double)l.z;
+    double acc = 0.0;
+    for (long long t = j_begin; t < j_end; t += kPotSub) {
+        __syncthreads();
+        if (tid < kPotSub && t + tid < j_end) {
+            const float4 q = pos[t + tid];
+            const float4 ql = plo ? plo[t + tid] : zero;
+            sx[tid] = (double)q.x + (double)ql.x;
+            sy[tid] = (double)q.y + (double)ql.y;
+            sz[tid] = (double)q.z + (double)ql.z;
+            smm[tid] = q.w;
+        }
+        __syncthreads();
+        const int kmax = (int)min((long long)kPotSub, j_end - t);
+#pragma unroll 4
+        for (int k = 0; k < kmax; ++k)
+            if (t + k > i) acc += smm[k] * pair_phi(sx[k] - xi, sy[k] - yi, sz[k] - zi, eps2, spline_h);
+    }
+    const double t = pot_block_sum(i < n ? -(double)p.w * acc : 0.0);
+    if (tid == 0) *out = t;
+}
+
+bool potential_scaled(long long n) { return n >= kPotDfMin; }
+
+void launch_potential(long long n, const Particles& P, bool split, double eps2, double spline_h, double mscale,
+                      double* partial, cudaStream_t s) {
+    const dim3 grid((unsigned)pot_tiles(n), (unsigned)pot_chunks(n));
+    const long long chunk = potential_chunk(n);
+    if (!potential_scaled(n))
+        potential_f64_kernel<<<grid, kPotThreads, 0, s>>>(n, P.pos, split ? P.plo : nullptr, eps2, spline_h, chunk,
+                                                          partial);
+    else if (split)
+        potential_df_kernel<true><<<grid, kPotThreads, 0, s>>>(n, P.pos, P.plo, eps2, spline_h, mscale, chunk, partial);
+    else
+        potential_df_kernel<false><<<grid, kPotThreads, 0, s>>>(n, P.pos, nullptr, eps2, spline_h, mscale, chunk,
+                                                                partial);
+}
+
+}  // namespace ngrav
