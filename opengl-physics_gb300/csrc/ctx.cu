@@ -155,7 +155,10 @@ int alloc_lists(ngrav_gpu_ctx* ctx, long long far_chunks, long long near_chunks)
 
 int alloc_group_info(ngrav_gpu_ctx* ctx, long long n) {
     dfree(ctx->LB.ginfo);
+    dfree(ctx->LB.passes);
     NG_CUDA(dalloc(ctx->LB.ginfo, std::max<long long>(n, 1)));
+    // passes past the first of leaves that hold at most n particles together
+    NG_CUDA(dalloc(ctx->LB.passes, n / kPassMin + 1));
     return NGRAV_OK;
 }
 
@@ -239,7 +242,7 @@ void enqueue_eval(ngrav_gpu_ctx* ctx, bool bbox_ready, bool kick, float hdt) {
                        s);
     launch_leaf_list(ctx->T, ctx->C, n, ctx->leaf_at, ctx->flags, ctx->scanbuf, ctx->leaf_list, ctx->SB, s);
     rec(ctx, 3);
-    launch_moments(ctx->T, ctx->C, P, ctx->leaf_list, n, (int)std::min<long long>(n, ctx->T.cap), split,
+    launch_moments(ctx->T, ctx->C, P, ctx->leaf_list, ctx->LB, n, (int)std::min<long long>(n, ctx->T.cap), split,
                    ctx->opts.quadrupole != 0, levels, s);
     rec(ctx, 4);
     WalkParams wp = walk_params(ctx, kick, hdt);
@@ -598,7 +601,6 @@ int ngrav_gpu_create(ngrav_gpu_ctx** out, const ngrav_gpu_opts* opts) {
         NG_CUDA(cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, ctx->opts.device));
         NG_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
         NG_CUDA(cudaMalloc((void**)&ctx->C, sizeof(Counters)));
-        eval_set_attributes();
         lmac_set_attributes();
         NG_CUDA(cudaGetLastError());
         // Walk: up to 32 resident warps per SM (latency-bound traversal);
@@ -638,6 +640,7 @@ void ngrav_gpu_destroy(ngrav_gpu_ctx* ctx) {
     dfree(ctx->LB.far_next);
     dfree(ctx->LB.near_next);
     dfree(ctx->LB.ginfo);
+    dfree(ctx->LB.passes);
     dfree(ctx->dpartial);
     dfree(ctx->dtargets);
     dfree(ctx->dslots);

@@ -39,13 +39,11 @@ int sampler_shares(long long n, int nslots, int sm_count);
 void launch_sampler(long long n, const Particles& P, bool split, const int* slots, int nslots, double eps2,
                     double spline_h, bool fp64_pairs, double* out, double* partial, int shares, cudaStream_t s);
 void launch_reset_counters(Counters* C, cudaStream_t s);
-void eval_set_attributes();
 void lmac_set_attributes();
 int walk_warps_per_block();
 int walk_blocks_per_sm();
 int eval_warps_per_block();
 int eval_blocks_per_sm();
-size_t eval_smem_bytes();
 void launch_gather_slots(const int* inv, const int* targets, int nt, int* slots, cudaStream_t s);
 double run_fma_probe(int sm_count, cudaStream_t s);
 

@@ -61,7 +61,7 @@ struct Counters {
     int work_next;                    // dynamic group scheduler (walk)
     int stack_max;
     int levels_used;
-    int eval_next;                    // dynamic group scheduler (evaluation)
+    int eval_next;                    // dynamic pass scheduler (evaluation)
     double root_center[3];
     double root_half;
     unsigned long long far_total;     // list entries written (far, near)
@@ -69,7 +69,7 @@ struct Counters {
     int list_max;                     // longest per-group list seen
     int far_chunks;                   // chunk allocators (may exceed the pool: then
     int near_chunks;                  //   they count what a retry needs)
-    int pad2;
+    int extra_passes;                 // evaluation passes past each group's first (ListBuffers::passes)
     // learned opening test: pairs handed to the network, accepted by it, and
     // decided by the geometric fallback (low confidence); tensor-core flushes
     unsigned long long lm_queries;
@@ -79,6 +79,20 @@ struct Counters {
     unsigned long long lm_screened;   // band pairs the error bound accepted without the network
     unsigned long long targets;       // particles whose acceleration a block-step evaluation refreshed
 };
+
+// Targets per pass of the evaluation (eval.cu).  A pass (of one group) is the
+// unit of work of a warp.  A pass of more targets loads the group's lists fewer
+// times, so the largest is taken where the groups alone fill the GPU's 152 x 16
+// warps four times over, and smaller ones below that, where idle warps and
+// long units cost more.  Evaluation kernel, leaf capacity 64: 2,500 bodies
+// (spline) 356 us before, 121 at 20 targets a pass, 46 at 5; 150,000 bodies
+// 2.97 ms before, 3.54 with a group's passes on one warp, 2.37 as units.  The
+// choice changes no sum.
+constexpr int kPassMax = 20, kPassMid = 10, kPassMin = 5;
+constexpr int kEvalWave = 152 * 16;
+__host__ __device__ inline int pass_targets(int groups) {
+    return groups >= 4 * kEvalWave ? kPassMax : (groups >= kEvalWave ? kPassMid : kPassMin);
+}
 
 // Per-group interaction lists written by the walk, read by the evaluation.
 // Each list is a chain of kListChunk-entry chunks taken from a pool with one
@@ -91,6 +105,7 @@ struct ListBuffers {
     int* far_next = nullptr;          // chunk links
     int* near_next = nullptr;
     int4* ginfo = nullptr;            // per group: far first chunk, near first chunk, far count, near count
+    int2* passes = nullptr;           // evaluation passes past each group's first: group, pass (n / kPassMin entries)
     int* stack = nullptr;             // per walking warp traversal stack
     int stack_cap = 0;
     int nwarps = 0;                   // resident walking warps
@@ -123,8 +138,8 @@ struct NodeArrays {
     float4* wB = nullptr;             // Qxx, Qyy, Qxy, Qxz
     float4* wC = nullptr;             // maxR (rounded up), 2h, link (int bits), meta (int bits)
     float4* wD = nullptr;             // com_lo.xyz, Qyz
-    float4* chi = nullptr;            // centre hi (leaves; SPLIT)
-    float4* clo = nullptr;            // centre lo (leaves; SPLIT)
+    float4* chi = nullptr;            // leaves: centre hi, first slot (int bits)
+    float4* clo = nullptr;            // leaves: centre lo, particle count (int bits)
 };
 
 // wC.w meta: bit 31 leaf flag; bits 0..23 count (leaf) or nchild (internal);
@@ -182,7 +197,7 @@ struct WalkParams {
     int smem_stack;                   // per-warp shared-memory walk stack: 1024, 2048 or 4096 entries
     int soft;                         // kSoftPlummer or kSoftSpline (softening.cuh)
     float ih;                         // spline: 1 / h (h = eps)
-    int p2p_tile;                     // sources per near batch of the evaluation (64..256; 0: 256)
+    int p2p_tile;                     // sources per near batch of the evaluation (64, 128, 256; 0: its maximum)
     // learned opening test (walk_lmac_kernel)
     int learned;
     float lm_log2b;                   // log2 of the per-target error budget
@@ -273,8 +288,9 @@ void launch_tree_levels(NodeArrays& T, Counters* C, const unsigned long long* ke
                         int max_depth, const Forest& F, int levels, cudaStream_t s);
 void launch_leaf_list(NodeArrays& T, Counters* C, long long n, int* leaf_at, unsigned* flags, unsigned* scan_out,
                       int* leaf_list, SortBuffers& sb, cudaStream_t s);
-void launch_moments(NodeArrays& T, Counters* C, const Particles& P, const int* leaf_list, long long n,
-                    int max_leaves, bool split, bool quadrupole, int levels, cudaStream_t s);
+// Leaf and internal moments; also the evaluation's pass list (LB.passes).
+void launch_moments(NodeArrays& T, Counters* C, const Particles& P, const int* leaf_list, const ListBuffers& LB,
+                    long long n, int max_leaves, bool split, bool quadrupole, int levels, cudaStream_t s);
 void launch_walk(const NodeArrays& T, Counters* C, const int* leaf_list, const WalkParams& wp,
                  const ListBuffers& LB, cudaStream_t s);
 void launch_eval(const NodeArrays& T, Counters* C, const Particles& P, const int* leaf_list, const WalkParams& wp,

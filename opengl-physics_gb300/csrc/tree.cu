@@ -318,12 +318,19 @@ __device__ __forceinline__ void df_add_prod(float& Sh, float& Sl, float m, float
 __global__ void __launch_bounds__(128) moments_kernel(NodeArrays T, Counters* C, const float4* __restrict__ pos,
                                                       const float4* __restrict__ plo, float4* __restrict__ src,
                                                       const float4* __restrict__ acc,
-                                                      const int* __restrict__ leaf_list, int split, int quadrupole) {
+                                                      const int* __restrict__ leaf_list, int2* __restrict__ passes,
+                                                      int split, int quadrupole) {
     const int nleaves = C->nleaves;
+    const int pass = pass_targets(nleaves);
     const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int li = blockIdx.x * blockDim.x + threadIdx.x; li < nleaves; li += gridDim.x * blockDim.x) {
         const int leaf = leaf_list[li];
         const int s = T.start[leaf], cnt = T.count[leaf];
+        if (cnt > pass) {
+            const int more = (cnt - 1) / pass;
+            const int at = atomicAdd(&C->extra_passes, more);
+            for (int p = 0; p < more; ++p) passes[at + p] = make_int2(li, p + 1);
+        }
         const double ccx = T.cx[leaf], ccy = T.cy[leaf], ccz = T.cz[leaf];
         const float chx = (float)ccx, chy = (float)ccy, chz = (float)ccz;
         const float clx = (float)(ccx - (double)chx), cly = (float)(ccy - (double)chy),
@@ -414,8 +421,8 @@ __global__ void __launch_bounds__(128) moments_kernel(NodeArrays T, Counters* C,
         for (int k = 0; k < 5; ++k) T.quad[5 * leaf + k] = Q[k];
         const int level = T.level[leaf];
         write_walk_record(T, leaf, M, cx, cy, cz, Q, maxr, true, s, cnt, level);
-        T.chi[leaf] = make_float4(chx, chy, chz, 0.f);
-        T.clo[leaf] = make_float4(clx, cly, clz, 0.f);
+        T.chi[leaf] = make_float4(chx, chy, chz, __int_as_float(s));
+        T.clo[leaf] = make_float4(clx, cly, clz, __int_as_float(cnt));
     }
 }
 
@@ -513,13 +520,13 @@ __global__ void __launch_bounds__(256) internal_moments_kernel(NodeArrays T, con
     }
 }
 
-void launch_moments(NodeArrays& T, Counters* C, const Particles& P, const int* leaf_list, long long n,
-                    int max_leaves, bool split, bool quadrupole, int levels, cudaStream_t s) {
+void launch_moments(NodeArrays& T, Counters* C, const Particles& P, const int* leaf_list, const ListBuffers& LB,
+                    long long n, int max_leaves, bool split, bool quadrupole, int levels, cudaStream_t s) {
     long long blocks = ((long long)max_leaves + 127) / 128;
     if (blocks > 152 * 16) blocks = 152 * 16;
     if (blocks < 1) blocks = 1;
     moments_kernel<<<(unsigned)blocks, 128, 0, s>>>(T, C, P.pos, split ? P.plo : nullptr, P.src, P.acc, leaf_list,
-                                                    split ? 1 : 0, quadrupole ? 1 : 0);
+                                                    LB.passes, split ? 1 : 0, quadrupole ? 1 : 0);
     long long b2 = ((long long)T.cap / 4 + 255) / 256;
     if (b2 > 152 * 4) b2 = 152 * 4;
     if (b2 < 1) b2 = 1;
