@@ -253,7 +253,8 @@ void enqueue_eval(ngrav_gpu_ctx* ctx, bool bbox_ready, bool kick, float hdt) {
         // (ComputeAccelBarnesHutTargets, Solvers.cpp:384-405)
         rec(ctx, 5);
         launch_walk_pp(ctx->T, ctx->C, P, ctx->leaf_list, wp, ctx->block_on ? 0 : 1, ctx->alpha, nullptr,
-                       ctx->block_on ? ctx->block_args : nullptr, ctx->block_base, ctx->LB.nwarps, s);
+                       ctx->block_on ? ctx->block_args : nullptr, ctx->block_base, n, ctx->scanbuf, ctx->flags,
+                       ctx->LB.nwarps, s);
         rec(ctx, 6);
         ctx->launches += 1;
         return;
@@ -602,6 +603,7 @@ int ngrav_gpu_create(ngrav_gpu_ctx** out, const ngrav_gpu_opts* opts) {
         NG_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
         NG_CUDA(cudaMalloc((void**)&ctx->C, sizeof(Counters)));
         lmac_set_attributes();
+        walk_pp_set_attributes();
         NG_CUDA(cudaGetLastError());
         // Walk: up to 32 resident warps per SM (latency-bound traversal);
         // evaluation: every warp the occupancy calculator allows.
