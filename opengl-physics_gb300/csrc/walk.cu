@@ -18,9 +18,10 @@
 //      a += -G Q.d / r^5 + 2.5 G (d.Q.d) d / r^7  (AddQuadrupole, :147-179).
 //
 // Walk: one warp per group, groups taken dynamically in key order.  Each
-// iteration tests up to 64 nodes (two per lane); near leaves and far nodes
-// are appended (ballot + prefix) to the group's lists with coalesced stores,
-// opened children are pushed on a per-warp stack.  The
+// iteration takes up to 4 kNPL opened nodes off a per-warp stack and tests
+// their children (lane = child, kNPL per lane); near leaves and far nodes are
+// appended (ballot + prefix) to the group's lists with coalesced stores, opened
+// nodes are pushed.  The
 // opening test runs in FP32 on double-float COMs; decisions within a
 // relative band of 1e-5 of the threshold are re-taken in FP64 on the FP64
 // moments.  Lists are chains of 128-entry chunks taken from a pool with one
@@ -38,25 +39,35 @@ namespace ngrav {
 
 constexpr int kWalkWarps = 4;
 constexpr int kWalkThreads = kWalkWarps * 32;
-constexpr int kNPL = 2;  // nodes tested per lane per iteration (memory-level parallelism)
+// Nodes tested per lane per iteration, their loads in flight together.  The
+// walk is bound by instruction issue and by the latency of one iteration (the
+// records come from the L2), so an iteration's cost is what counts: with a
+// stack of opened nodes instead of one of nodes to test, a push is one store per
+// opened node without a prefix sum, and siblings are read as whole lines.  1 Mi
+// bodies (theta 0.5, plain): 3.50 ms with nodes on the stack, 2.86 ms so; 4 Mi
+// (theta 1): 3.72 and 2.86 ms.  One, three and four per lane were all slower.
+constexpr int kNPL = 2;
 
-// STACK > 0: a per-warp traversal stack of STACK entries in shared memory
-// (push -> pop never leaves the SM; the size trades occupancy against the
-// frontier it holds, a tuned choice); STACK = 0: the global-memory stack, the
-// fallback for trees whose frontier outgrows shared memory.
+// STACK > 0: a per-warp traversal stack for a frontier of STACK nodes in shared
+// memory (STACK / 4 opened nodes; push -> pop never leaves the SM, the size
+// trades L1 and occupancy against the frontier it holds, a tuned choice);
+// STACK = 0: the global-memory stack, the fallback for trees whose frontier
+// outgrows shared memory.
 template <int STACK>
 __global__ void __launch_bounds__(kWalkThreads) walk_kernel(NodeArrays T, Counters* C,
                                                             const int* __restrict__ leaf_list, WalkParams wp,
                                                             ListBuffers LB) {
-    __shared__ int s_stack[STACK > 0 ? kWalkWarps * STACK : 1];
+    __shared__ int2 s_stack[STACK > 0 ? kWalkWarps * STACK / 4 : 1];
     const int lane = threadIdx.x & 31;
     const int gwarp = blockIdx.x * kWalkWarps + (threadIdx.x >> 5);
     if (C->status & kStFatal) return;
-    int* stack = STACK > 0 ? s_stack + (threadIdx.x >> 5) * STACK : LB.stack + (long long)gwarp * LB.stack_cap;
-    const int stack_cap = STACK > 0 ? STACK : LB.stack_cap;
+    int2* stack = STACK > 0 ? s_stack + (threadIdx.x >> 5) * (STACK / 4)
+                            : reinterpret_cast<int2*>(LB.stack + (long long)gwarp * LB.stack_cap);
+    const int stack_cap = STACK > 0 ? STACK / 4 : LB.stack_cap / 2;
     const int nleaves = C->nleaves;
     const unsigned lt_mask = (1u << lane) - 1u;
-    unsigned long long tests = 0, retests = 0, groups = 0;
+    unsigned tests = 0, retests = 0;                              // of this lane
+    unsigned long long groups = 0;
     int stack_max = 0, list_max = 0;
     unsigned bad = 0;
     int fres_next = 0, fres_end = 0, nres_next = 0, nres_end = 0;  // chunk reservoirs
@@ -83,16 +94,13 @@ __global__ void __launch_bounds__(kWalkThreads) walk_kernel(NodeArrays T, Counte
         // own members first (the self term is zero)
         list_append(near, lane == 0, leaf, LB.near, LB.near_next, &C->near_chunks, LB.near_chunk_cap, lane,
                     lt_mask, bad);
-        int size = 0, visits = 0;
+        int size = 0, iterations = 0;
         const int root = T.sysroot[leaf];
         if (leaf != root) {
             // The root's test, by every lane at once (the same arithmetic as
-            // the loop's): when it opens, as it nearly always does, its
-            // children start the stack, sparing an iteration that would test
-            // one node; otherwise the root takes the loop's path.
+            // the loop's, which tests the children of opened nodes).
             const float4 A = T.wA[root], Cw = T.wC[root], D = T.wD[root];
             const int meta = __float_as_int(Cw.w);
-            bool open = false;
             if (A.w > 0.f && meta >= 0) {
                 const float dx = (A.x - gA.x) + (D.x - gD.x);
                 const float dy = (A.y - gA.y) + (D.y - gD.y);
@@ -113,110 +121,87 @@ __global__ void __launch_bounds__(kWalkThreads) walk_kernel(NodeArrays T, Counte
                         accept = w > 0.0 && sz * sz < wp.theta2_d * w * w;
                     }
                 }
-                open = !accept;
-            }
-            if (open) {
-                const int nch = meta & 0xFFFFFF, link = __float_as_int(Cw.z);
-                if (lane < nch) stack[lane] = link + lane;
-                size = nch;
-                visits = 1;
-                tests += 1;
-            } else {
-                if (lane == 0) stack[0] = root;
-                size = 1;
+                if (lane == 0) ++tests;
+                if (accept) {
+                    list_append(far, lane == 0, root, LB.far, LB.far_next, &C->far_chunks, LB.far_chunk_cap, lane,
+                                lt_mask, bad);
+                } else {
+                    if (lane == 0) stack[0] = make_int2(__float_as_int(Cw.z), meta & 0xFFFFFF);
+                    size = 1;
+                }
             }
         }
         __syncwarp();
         while (size > 0) {
-            const int take = min(size, 32 * kNPL);
+            const int take = min(size, 4 * kNPL);  // opened nodes; lane = child
             size -= take;
-            visits += take;
-            if (visits > wp.node_limit) {
-                bad |= kStCorrupt;
-                break;
-            }
             int node[kNPL];
 #pragma unroll
             for (int q = 0; q < kNPL; ++q) {
-                const int idx = lane + 32 * q;
-                node[q] = idx < take ? stack[size + idx] : -1;
+                const int p = 4 * q + (lane >> 3);
+                const int2 e = p < take ? stack[size + p] : make_int2(0, 0);
+                // a lane without a child reads the group's own leaf, which the tests skip
+                node[q] = (lane & 7) < e.y ? e.x + (lane & 7) : leaf;
+            }
+            if (++iterations > wp.node_limit) {  // every iteration opens a node of its own
+                bad |= kStCorrupt;
+                break;
             }
             float4 A[kNPL], Cw[kNPL], Dw[kNPL];
 #pragma unroll
             for (int q = 0; q < kNPL; ++q) {  // all record loads in flight together
-                if (node[q] >= 0) {
-                    A[q] = T.wA[node[q]];
-                    Cw[q] = T.wC[node[q]];
-                    Dw[q] = T.wD[node[q]];
-                } else {
-                    A[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    Cw[q] = A[q];
-                    Dw[q] = A[q];
-                }
+                A[q] = T.wA[node[q]];
+                Cw[q] = T.wC[node[q]];
+                Dw[q] = T.wD[node[q]];
             }
-            int kind[kNPL], nch[kNPL], link[kNPL];
-            bool tested_any[kNPL];
+            bool near_k[kNPL], far_k[kNPL], open_k[kNPL];
+            int nch[kNPL], link[kNPL];
 #pragma unroll
             for (int q = 0; q < kNPL; ++q) {
-                kind[q] = 0;  // 0 none, 1 near, 2 far, 3 open
-                nch[q] = 0;
-                tested_any[q] = false;
                 const int meta = __float_as_int(Cw[q].w);
                 link[q] = __float_as_int(Cw[q].z);
-                if (node[q] >= 0 && node[q] != leaf && A[q].w > 0.f) {
-                    if (meta < 0) {
-                        kind[q] = 1;
-                    } else {
-                        tested_any[q] = true;
-                        const float4 D = Dw[q];
-                        const float dx = (A[q].x - gA.x) + (D.x - gD.x);
-                        const float dy = (A[q].y - gA.y) + (D.y - gD.y);
-                        const float dz = (A[q].z - gA.z) + (D.z - gD.z);
-                        const float dist = sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
-                        const float worst = dist - gR;
-                        const float size_n = Cw[q].y;
-                        bool accept = worst > 0.f && size_n * size_n < wp.theta2 * worst * worst;
-                        if (wp.retest) {
-                            const float margin = wp.theta * worst - size_n;
-                            if (fabsf(margin) <= 1e-5f * (wp.theta * (dist + gR) + size_n)) {
-                                ++retests;
-                                const int nd = node[q];
-                                const double ex = T.comx[nd] - gcx_d, ey = T.comy[nd] - gcy_d,
-                                             ez = T.comz[nd] - gcz_d;
-                                const double d2 = ex * ex + ey * ey + ez * ez;
-                                const double sz = 2.0 * T.half[nd];
-                                const double w = sqrt(d2) - gr_d;
-                                accept = w > 0.0 && sz * sz < wp.theta2_d * w * w;
-                            }
-                        }
-                        if (accept) {
-                            kind[q] = 2;
-                        } else {
-                            kind[q] = 3;
-                            nch[q] = meta & 0xFFFFFF;
-                        }
+                nch[q] = meta & 0xFFFFFF;
+                const bool massive = node[q] != leaf && A[q].w > 0.f;
+                const bool inner = massive && meta >= 0;
+                near_k[q] = massive && meta < 0;
+                tests += inner ? 1u : 0u;
+                const float4 D = Dw[q];
+                const float dx = (A[q].x - gA.x) + (D.x - gD.x);
+                const float dy = (A[q].y - gA.y) + (D.y - gD.y);
+                const float dz = (A[q].z - gA.z) + (D.z - gD.z);
+                const float dist = sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
+                const float worst = dist - gR;
+                const float size_n = Cw[q].y;
+                bool accept;
+                if (wp.retest) {
+                    // outside the band the margin's sign is the test's outcome
+                    const float margin = wp.theta * worst - size_n;
+                    accept = margin > 0.f;
+                    if (inner && fabsf(margin) <= 1e-5f * (wp.theta * (dist + gR) + size_n)) {
+                        ++retests;
+                        const int nd = node[q];
+                        const double ex = T.comx[nd] - gcx_d, ey = T.comy[nd] - gcy_d, ez = T.comz[nd] - gcz_d;
+                        const double d2 = ex * ex + ey * ey + ez * ez;
+                        const double sz = 2.0 * T.half[nd];
+                        const double w = sqrt(d2) - gr_d;
+                        accept = w > 0.0 && sz * sz < wp.theta2_d * w * w;
                     }
+                } else {
+                    accept = worst > 0.f && size_n * size_n < wp.theta2 * worst * worst;
                 }
+                far_k[q] = inner && accept;
+                open_k[q] = inner && !accept;
             }
-            static_assert(kNPL == 2, "the batched appends below take two nodes per lane");
-            tests += __popc(__ballot_sync(0xffffffffu, tested_any[0])) +
-                     __popc(__ballot_sync(0xffffffffu, tested_any[1]));
-            list_append2(near, kind[0] == 1, node[0], kind[1] == 1, node[1], LB.near, LB.near_next, &C->near_chunks,
-                         LB.near_chunk_cap, lane, lt_mask, bad);
-            list_append2(far, kind[0] == 2, node[0], kind[1] == 2, node[1], LB.far, LB.far_next, &C->far_chunks,
-                         LB.far_chunk_cap, lane, lt_mask, bad);
-            {  // both nodes' children onto the stack with one scan
-                int tot;
-                const int off = warp_excl_scan(nch[0] + nch[1], lane, tot);
-                if (size + tot > stack_cap) {
-                    bad |= kStStackOverflow;
-                    break;
-                }
-                for (int k = 0; k < nch[0]; ++k) stack[size + off + k] = link[0] + k;
-                for (int k = 0; k < nch[1]; ++k) stack[size + off + nch[0] + k] = link[1] + k;
-                size += tot;
+            list_append_n<kNPL>(near, near_k, node, LB.near, LB.near_next, &C->near_chunks, LB.near_chunk_cap, lane,
+                                lt_mask, bad);
+            list_append_n<kNPL>(far, far_k, node, LB.far, LB.far_next, &C->far_chunks, LB.far_chunk_cap, lane,
+                                lt_mask, bad);
+            __syncwarp();  // the entries above were read by every lane
+            if (!push_opened<kNPL>(stack, size, stack_cap, open_k, link, nch, lt_mask)) {
+                bad |= kStStackOverflow;
+                break;
             }
-            stack_max = max(stack_max, size);
+            stack_max = max(stack_max, 4 * size);
             __syncwarp();
         }
         fres_next = far.res_next;
@@ -227,16 +212,20 @@ __global__ void __launch_bounds__(kWalkThreads) walk_kernel(NodeArrays T, Counte
         list_max = max(list_max, max(far.count, near.count));
         if (bad & (kStStackOverflow | kStCorrupt)) break;
     }
-    for (int o = 16; o > 0; o >>= 1) bad |= __shfl_xor_sync(0xffffffffu, bad, o);
+    unsigned long long all_tests = tests, all_retests = retests;
+    for (int o = 16; o > 0; o >>= 1) {
+        bad |= __shfl_xor_sync(0xffffffffu, bad, o);
+        all_tests += __shfl_xor_sync(0xffffffffu, all_tests, o);
+        all_retests += __shfl_xor_sync(0xffffffffu, all_retests, o);
+    }
     if (lane == 0) {
         if (bad) atomicOr(&C->status, bad);
-        atomicAdd(&C->mac_tests, tests);
+        atomicAdd(&C->mac_tests, all_tests);
         atomicAdd(&C->groups, groups);
         atomicMax(&C->stack_max, stack_max);
         atomicMax(&C->list_max, list_max);
     }
-    for (int o = 16; o > 0; o >>= 1) retests += __shfl_xor_sync(0xffffffffu, retests, o);
-    if (lane == 0 && retests) atomicAdd(&C->mac_retests, retests);
+    if (lane == 0 && all_retests) atomicAdd(&C->mac_retests, all_retests);
 }
 
 // ---------------------------------------------------------------------------

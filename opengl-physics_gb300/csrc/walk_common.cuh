@@ -71,36 +71,45 @@ __device__ __forceinline__ void list_append(ChunkList& L, bool has, int val, int
     L.count += k;
 }
 
-// Two candidates per lane (v0 then v1), appended as one batch of up to 64:
-// all v0 in lane order, then all v1.  One chunk-boundary check for both.
-__device__ __forceinline__ void list_append2(ChunkList& L, bool has0, int v0, bool has1, int v1,
-                                             int* __restrict__ pool, int* __restrict__ next, int* counter, int cap,
-                                             int lane, unsigned lt_mask, unsigned& bad) {
-    const unsigned m0 = __ballot_sync(0xffffffffu, has0);
-    const unsigned m1 = __ballot_sync(0xffffffffu, has1);
-    const int k0 = __popc(m0);
-    const int k = k0 + __popc(m1);
+// N candidates per lane, appended as one batch of up to 32 N <= kListChunk: all
+// of the first in lane order, then all of the next.  One chunk-boundary check
+// for all.
+template <int N>
+__device__ __forceinline__ void list_append_n(ChunkList& L, const bool (&has)[N], const int (&val)[N],
+                                              int* __restrict__ pool, int* __restrict__ next, int* counter, int cap,
+                                              int lane, unsigned lt_mask, unsigned& bad) {
+    static_assert(32 * N <= kListChunk, "at most one new chunk");
+    unsigned m[N];
+    int k = 0;
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+        m[q] = __ballot_sync(0xffffffffu, has[q]);
+        k += __popc(m[q]);
+    }
     if (k == 0) return;
     if (L.cur < 0) {
         L.cur = L.first = alloc_chunk(L, counter, lane);
         L.pos = 0;
     }
     int newc = -1;
-    if (L.pos + k > kListChunk) {  // k <= 64 < kListChunk: at most one new chunk
+    if (L.pos + k > kListChunk) {
         newc = alloc_chunk(L, counter, lane);
         if (lane == 0 && L.cur < cap) next[L.cur] = newc;
     }
+    // entry i goes to the current chunk, or past its end to the new one
+    int* const cur = pool + (long long)L.cur * kListChunk;
+    int* const nxt = pool + ((long long)newc - 1) * kListChunk;
+    const bool cur_in = L.cur < cap, nxt_in = newc < cap;
+    if (!cur_in || !nxt_in) bad |= kStListOverflow;
+    int at = L.pos;
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        if (q == 0 ? has0 : has1) {
-            const int i = L.pos + (q == 0 ? __popc(m0 & lt_mask) : k0 + __popc(m1 & lt_mask));
-            const int c = i < kListChunk ? L.cur : newc;
-            const int p = i < kListChunk ? i : i - kListChunk;
-            if (c < cap)
-                pool[(long long)c * kListChunk + p] = q == 0 ? v0 : v1;
-            else
-                bad |= kStListOverflow;
+    for (int q = 0; q < N; ++q) {
+        if (has[q]) {
+            const int i = at + __popc(m[q] & lt_mask);
+            const bool here = i < kListChunk;
+            if (here ? cur_in : nxt_in) (here ? cur : nxt)[i] = val[q];
         }
+        at += __popc(m[q]);
     }
     if (newc >= 0) {
         L.cur = newc;
@@ -109,6 +118,32 @@ __device__ __forceinline__ void list_append2(ChunkList& L, bool has0, int v0, bo
         L.pos += k;
     }
     L.count += k;
+}
+
+// The walk stack holds opened nodes, as (first child, children): one store per
+// opened node instead of one per child, and an iteration takes four of them per
+// 32 lanes, lane = child, so a node's children are read as one 128-byte line
+// per record array.  Pushes the nodes with `open`, in lane order, then those of
+// the next set; false if they do not fit.
+template <int N>
+__device__ __forceinline__ bool push_opened(int2* stack, int& size, int cap, const bool (&open)[N],
+                                            const int (&link)[N], const int (&nch)[N], unsigned lt_mask) {
+    int at = size;
+    unsigned m[N];
+    int k = 0;
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+        m[q] = __ballot_sync(0xffffffffu, open[q]);
+        k += __popc(m[q]);
+    }
+    if (size + k > cap) return false;
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+        if (open[q]) stack[at + __popc(m[q] & lt_mask)] = make_int2(link[q], nch[q]);
+        at += __popc(m[q]);
+    }
+    size = at;
+    return true;
 }
 
 }  // namespace ngrav

@@ -29,18 +29,41 @@
 #include "lmac_tc.cuh"
 #include "walk_common.cuh"
 
+#include <utility>
+
 namespace ngrav {
 
 constexpr int kLwWarps = 4;
 constexpr int kLwThreads = kLwWarps * 32;
-// Per-warp shared-memory traversal stack: 2048 entries at 6 CTAs per SM, or
-// 1024 at 8 (the walk_stack tuning knob picks; an overflow moves the run to
-// the global-memory stack).
+// Per-warp shared-memory traversal stack: a frontier of 2048 nodes, with 7 CTAs
+// per SM, or of 1024 with 8 (the walk_stack tuning knob picks; an overflow moves
+// the run to the global-memory stack).  The kernel waits on the L2 for most of
+// its time, so the warps in flight count: the whole learned walk (three rounds
+// and two inferences) of 4 Mi / 16.8 M bodies took 3.33 / 14.85 ms with nodes on
+// the stack and 5 CTAs, and takes 2.64 / 12.08 ms with opened nodes (push_opened)
+// and 7; 6 CTAs were about 4 % slower than 7.
+
+// The pools of a round, as the kernels get them (round_pools): the one it
+// fills, and the one of the round before that it resolves.  Constant places,
+// because an index that varies puts the whole parameter struct into local
+// memory.
+constexpr int kOut = 0, kIn = 1;
+
+static LmacRounds round_pools(LmacRounds R, int round) {
+    if (round & 1) {
+        std::swap(R.active[0], R.active[1]);
+        std::swap(R.pend_node[0], R.pend_node[1]);
+        std::swap(R.pend_next[0], R.pend_next[1]);
+        std::swap(R.pend_owner[0], R.pend_owner[1]);
+        std::swap(R.pend_fill[0], R.pend_fill[1]);
+    }
+    return R;
+}
 
 // Append to a group's deferred-pair list: chunks taken one at a time (so
 // every chunk counted is owned and filled), owner and fill recorded for the
 // tensor-core kernel.
-__device__ __forceinline__ void pend_append(ChunkList& L, bool has, int val, const LmacRounds& R, int out,
+__device__ __forceinline__ void pend_append(ChunkList& L, bool has, int val, const LmacRounds& R,
                                             int* counter, int leaf, int lane, unsigned lt_mask, unsigned& bad) {
     const unsigned m = __ballot_sync(0xffffffffu, has);
     const int k = __popc(m);
@@ -50,7 +73,7 @@ __device__ __forceinline__ void pend_append(ChunkList& L, bool has, int val, con
         int c = 0;
         if (lane == 0) {
             c = atomicAdd(counter, 1);
-            if (c < cap) R.pend_owner[out][c] = leaf;
+            if (c < cap) R.pend_owner[kOut][c] = leaf;
         }
         L.cur = L.first = __shfl_sync(0xffffffffu, c, 0);
         L.pos = 0;
@@ -60,10 +83,10 @@ __device__ __forceinline__ void pend_append(ChunkList& L, bool has, int val, con
         if (lane == 0) {
             newc = atomicAdd(counter, 1);
             if (L.cur < cap) {
-                R.pend_next[out][L.cur] = newc;
-                R.pend_fill[out][L.cur] = kPendChunk;
+                R.pend_next[kOut][L.cur] = newc;
+                R.pend_fill[kOut][L.cur] = kPendChunk;
             }
-            if (newc < cap) R.pend_owner[out][newc] = leaf;
+            if (newc < cap) R.pend_owner[kOut][newc] = leaf;
         }
         newc = __shfl_sync(0xffffffffu, newc, 0);
     }
@@ -72,7 +95,7 @@ __device__ __forceinline__ void pend_append(ChunkList& L, bool has, int val, con
         const int c = i < kPendChunk ? L.cur : newc;
         const int p = i < kPendChunk ? i : i - kPendChunk;
         if (c < cap) {
-            R.pend_node[out][(long long)c * kPendChunk + p] = val;
+            R.pend_node[kOut][(long long)c * kPendChunk + p] = val;
         } else {
             bad |= kStPendOverflow;
         }
@@ -110,22 +133,24 @@ __global__ void __launch_bounds__(kLwThreads, MINB) walk_lmac_round_kernel(NodeA
                                                                         const int* __restrict__ leaf_list,
                                                                         WalkParams wp, ListBuffers LB, LmacRounds R,
                                                                         int round) {
-    // STACK = 0: the global-memory stack of LB
-    __shared__ int s_stack[STACK > 0 ? kLwWarps * STACK : 1];
+    // opened nodes (walk_common.cuh), for a frontier of STACK nodes; STACK = 0:
+    // the global-memory stack of LB
+    __shared__ int2 s_stack[STACK > 0 ? kLwWarps * STACK / 4 : 1];
     const int lane = threadIdx.x & 31;
     const int gwarp = blockIdx.x * kLwWarps + (threadIdx.x >> 5);
     if (C->status & kStFatal) return;
-    int* stack = STACK > 0 ? s_stack + (threadIdx.x >> 5) * STACK : LB.stack + (long long)gwarp * LB.stack_cap;
-    const int stack_cap = STACK > 0 ? STACK : LB.stack_cap;
+    int2* stack = STACK > 0 ? s_stack + (threadIdx.x >> 5) * (STACK / 4)
+                            : reinterpret_cast<int2*>(LB.stack + (long long)gwarp * LB.stack_cap);
+    const int stack_cap = STACK > 0 ? STACK / 4 : LB.stack_cap / 2;
     const bool last = round == R.rounds - 1;
-    const int in = (round + 1) & 1, out = round & 1;
     const int ngroups = round == 0 ? C->nleaves : R.ctr[4 * (round - 1) + 1];
     int* sched = R.ctr + 4 * round;
-    int* active_out = R.active[out];
+    int* active_out = R.active[kOut];
     int* pend_ctr = R.ctr + 4 * round + 2;
     const unsigned lt_mask = (1u << lane) - 1u;
     const float four_g = 4.f * wp.G;
-    unsigned long long tests = 0, groups = 0, resolved = 0, screened = 0;
+    unsigned tests = 0, screened = 0;  // of this lane
+    unsigned long long groups = 0;
     int stack_max = 0, list_max = 0;
     unsigned bad = 0;
     int fres_next = 0, fres_end = 0, nres_next = 0, nres_end = 0;
@@ -135,7 +160,7 @@ __global__ void __launch_bounds__(kLwThreads, MINB) walk_lmac_round_kernel(NodeA
         if (lane == 0) k = atomicAdd(sched, 1);
         k = __shfl_sync(0xffffffffu, k, 0);
         if (k >= ngroups) break;
-        const int gi = round == 0 ? k : R.active[in][k];
+        const int gi = round == 0 ? k : R.active[kIn][k];
         const int leaf = leaf_list[gi];
         const float4 gA = T.wA[leaf];
         const float4 gD = T.wD[leaf];
@@ -152,28 +177,22 @@ __global__ void __launch_bounds__(kLwThreads, MINB) walk_lmac_round_kernel(NodeA
                         lt_mask, bad);
             const int root = T.sysroot[leaf];
             if (leaf != root) {
-                // The root's first rule (open when worst <= 0 or 2h >= rho_hi
-                // worst), by every lane at once: when it opens, as it nearly
-                // always does, its children start the stack, sparing an
-                // iteration that would test one node; otherwise the root takes
-                // the loop's path.
+                // The root, by every lane at once: it opens under the first rule
+                // (worst <= 0 or 2h >= rho_hi worst), as it nearly always does;
+                // otherwise it takes the loop's path as an opened node's only
+                // child.
                 const float4 A = T.wA[root], Cw = T.wC[root], D = T.wD[root];
                 const int meta = __float_as_int(Cw.w);
-                bool open = false;
                 if (A.w > 0.f && meta >= 0) {
                     const float dx = (A.x - gA.x) + (D.x - gD.x);
                     const float dy = (A.y - gA.y) + (D.y - gD.y);
                     const float dz = (A.z - gA.z) + (D.z - gD.z);
                     const float worst = sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) - gR;
-                    open = !(worst > 0.f) || Cw.y >= wp.lm_rho_hi * worst;
-                }
-                if (open) {
-                    const int nch = meta & 0xFFFFFF, link = __float_as_int(Cw.z);
-                    if (lane < nch) stack[lane] = link + lane;
-                    size = nch;
-                    tests += 1;
-                } else {
-                    if (lane == 0) stack[0] = root;
+                    const bool open = !(worst > 0.f) || Cw.y >= wp.lm_rho_hi * worst;
+                    if (lane == 0) {
+                        stack[0] = open ? make_int2(__float_as_int(Cw.z), meta & 0xFFFFFF) : make_int2(root, 1);
+                        tests += open ? 1u : 0u;
+                    }
                     size = 1;
                 }
             }
@@ -191,7 +210,7 @@ __global__ void __launch_bounds__(kLwThreads, MINB) walk_lmac_round_kernel(NodeA
                 bool acc = false;
                 if (has) {
                     const long long slot = (long long)chunk * kPendChunk + e;
-                    node = R.pend_node[in][slot] & 0x7FFFFFFF;
+                    node = R.pend_node[kIn][slot] & 0x7FFFFFFF;
                     acc = R.dec[slot] != 0;
                     if (!acc) {
                         const float4 Cw = T.wC[node];
@@ -199,58 +218,50 @@ __global__ void __launch_bounds__(kLwThreads, MINB) walk_lmac_round_kernel(NodeA
                         link = __float_as_int(Cw.z);
                     }
                 }
-                resolved += __popc(__ballot_sync(0xffffffffu, has));
                 list_append(far, has && acc, node, LB.far, LB.far_next, &C->far_chunks, LB.far_chunk_cap, lane,
                             lt_mask, bad);
-                int tot;
-                const int off = warp_excl_scan(nch, lane, tot);
-                if (size + tot > stack_cap) {
+                const bool opened[1] = {has && !acc};
+                const int links[1] = {link}, nchs[1] = {nch};
+                if (!push_opened<1>(stack, size, stack_cap, opened, links, nchs, lt_mask)) {
                     bad |= kStStackOverflow;
                     break;
                 }
-                for (int q = 0; q < nch; ++q) stack[size + off + q] = link + q;
-                size += tot;
-                if (((i0 + 32) & (kPendChunk - 1)) == 0 && i0 + 32 < g.pend_count) chunk = R.pend_next[in][chunk];
+                if (((i0 + 32) & (kPendChunk - 1)) == 0 && i0 + 32 < g.pend_count) chunk = R.pend_next[kIn][chunk];
             }
             __syncwarp();
         }
-        int visits = 0;
+        int iterations = 0;
         while (size > 0 && !(bad & (kStStackOverflow | kStCorrupt))) {
-            const int take = min(size, 64);
+            const int take = min(size, 8);  // opened nodes; lane = child, two per lane
             size -= take;
-            visits += take;
-            if (visits > wp.node_limit) {
+            if (++iterations > wp.node_limit) {
                 bad |= kStCorrupt;
                 break;
             }
             int node[2];
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const int idx = lane + 32 * q;
-                node[q] = idx < take ? stack[size + idx] : -1;
-            }
             float4 A[2], Cw[2], D[2];
 #pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int p = 4 * q + (lane >> 3);
+                const int2 e = p < take ? stack[size + p] : make_int2(0, 0);
+                // a lane without a child reads the group's own leaf, which is skipped
+                node[q] = (lane & 7) < e.y ? e.x + (lane & 7) : leaf;
+            }
+#pragma unroll
             for (int q = 0; q < 2; ++q) {  // every record in flight at once
-                if (node[q] >= 0) {
-                    A[q] = T.wA[node[q]];
-                    Cw[q] = T.wC[node[q]];
-                    D[q] = T.wD[node[q]];
-                } else {
-                    A[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    Cw[q] = A[q];
-                    D[q] = A[q];
-                }
+                A[q] = T.wA[node[q]];
+                Cw[q] = T.wC[node[q]];
+                D[q] = T.wD[node[q]];
             }
             __syncwarp();
             int kind[2], nch[2], link[2];
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 kind[q] = 0;  // 0 none, 1 near, 2 far, 3 open, 4 deferred
-                nch[q] = 0;
                 link[q] = __float_as_int(Cw[q].z);
                 const int meta = __float_as_int(Cw[q].w);
-                if (node[q] >= 0 && node[q] != leaf && A[q].w > 0.f) {
+                nch[q] = meta & 0xFFFFFF;
+                if (node[q] != leaf && A[q].w > 0.f) {
                     if (meta < 0) {
                         kind[q] = 1;
                     } else {
@@ -276,33 +287,24 @@ __global__ void __launch_bounds__(kLwThreads, MINB) walk_lmac_round_kernel(NodeA
                                 ++screened;
                             }
                         }
-                        if (kind[q] == 3) nch[q] = meta & 0xFFFFFF;
                         // the geometric decision rides in the deferred node id's top
                         // bit for the low-confidence fallback
                         if (kind[q] == 4 && sz * sz < wp.theta2 * worst * worst) node[q] |= (int)0x80000000u;
                     }
                 }
             }
-            tests += __popc(__ballot_sync(0xffffffffu, kind[0] >= 2)) + __popc(__ballot_sync(0xffffffffu, kind[1] >= 2));
-            list_append2(near, kind[0] == 1, node[0], kind[1] == 1, node[1], LB.near, LB.near_next, &C->near_chunks,
-                         LB.near_chunk_cap, lane, lt_mask, bad);
-            list_append2(far, kind[0] == 2, node[0], kind[1] == 2, node[1], LB.far, LB.far_next, &C->far_chunks,
-                         LB.far_chunk_cap, lane, lt_mask, bad);
+            tests += (kind[0] >= 2 ? 1u : 0u) + (kind[1] >= 2 ? 1u : 0u);
+            const bool near_k[2] = {kind[0] == 1, kind[1] == 1}, far_k[2] = {kind[0] == 2, kind[1] == 2};
+            const bool open_k[2] = {kind[0] == 3, kind[1] == 3};
+            list_append_n<2>(near, near_k, node, LB.near, LB.near_next, &C->near_chunks, LB.near_chunk_cap, lane,
+                             lt_mask, bad);
+            list_append_n<2>(far, far_k, node, LB.far, LB.far_next, &C->far_chunks, LB.far_chunk_cap, lane, lt_mask,
+                             bad);
 #pragma unroll
             for (int q = 0; q < 2; ++q)
-                pend_append(pend, kind[q] == 4, node[q], R, out, pend_ctr, leaf, lane, lt_mask, bad);
-            {  // both nodes' children onto the stack with one scan
-                int tot;
-                const int off = warp_excl_scan(nch[0] + nch[1], lane, tot);
-                if (size + tot > stack_cap) {
-                    bad |= kStStackOverflow;
-                } else {
-                    for (int c = 0; c < nch[0]; ++c) stack[size + off + c] = link[0] + c;
-                    for (int c = 0; c < nch[1]; ++c) stack[size + off + nch[0] + c] = link[1] + c;
-                    size += tot;
-                }
-            }
-            stack_max = max(stack_max, size);
+                pend_append(pend, kind[q] == 4, node[q], R, pend_ctr, leaf, lane, lt_mask, bad);
+            if (!push_opened<2>(stack, size, stack_cap, open_k, link, nch, lt_mask)) bad |= kStStackOverflow;
+            stack_max = max(stack_max, 4 * size);
             __syncwarp();
         }
         fres_next = far.res_next;
@@ -312,7 +314,7 @@ __global__ void __launch_bounds__(kLwThreads, MINB) walk_lmac_round_kernel(NodeA
         if (pend.count > 0) {
             // park the group until the network has decided its pairs
             if (lane == 0) {
-                if (pend.cur < R.pend_chunk_cap) R.pend_fill[out][pend.cur] = pend.pos;
+                if (pend.cur < R.pend_chunk_cap) R.pend_fill[kOut][pend.cur] = pend.pos;
                 LmacGroupState g;
                 g.far_first = far.first;
                 g.far_cur = far.cur;
@@ -334,19 +336,20 @@ __global__ void __launch_bounds__(kLwThreads, MINB) walk_lmac_round_kernel(NodeA
         }
         if (bad & (kStStackOverflow | kStCorrupt)) break;
     }
+    unsigned long long all_tests = tests, all_screened = screened;
     for (int o = 16; o > 0; o >>= 1) {
         bad |= __shfl_xor_sync(0xffffffffu, bad, o);
-        screened += __shfl_xor_sync(0xffffffffu, screened, o);
+        all_tests += __shfl_xor_sync(0xffffffffu, all_tests, o);
+        all_screened += __shfl_xor_sync(0xffffffffu, all_screened, o);
     }
     if (lane == 0) {
         if (bad) atomicOr(&C->status, bad);
-        atomicAdd(&C->mac_tests, tests);
-        if (screened) atomicAdd(&C->lm_screened, screened);
+        atomicAdd(&C->mac_tests, all_tests);
+        if (all_screened) atomicAdd(&C->lm_screened, all_screened);
         if (groups) atomicAdd(&C->groups, groups);
         atomicMax(&C->stack_max, stack_max);
         atomicMax(&C->list_max, list_max);
     }
-    (void)resolved;
 }
 
 // Decide every deferred pair of `round`: chunks 8t .. 8t+7 form tile t
@@ -366,15 +369,14 @@ __global__ void __launch_bounds__(kLwThreads) lmac_infer_kernel(NodeArrays T, Co
     if (threadIdx.x == 0) s_status = C->status;
     __syncthreads();
     if (s_status & kStFatal) return;  // uniform across the CTA
-    const int pool = round & 1;
     int nchunks = R.ctr[4 * round + 2];
     nchunks = nchunks < R.pend_chunk_cap ? nchunks : R.pend_chunk_cap;
     const int ntiles = (nchunks + 7) / 8;  // a tile: 8 chunks, two per warp
     if ((int)blockIdx.x >= ntiles) return;
     lmac_tc_init(S, model);
-    const int* pnode = R.pend_node[pool];
-    const int* fill = R.pend_fill[pool];
-    const int* owner = R.pend_owner[pool];
+    const int* pnode = R.pend_node[kOut];
+    const int* fill = R.pend_fill[kOut];
+    const int* owner = R.pend_owner[kOut];
     const float eps = sqrtf(wp.eps2);
     unsigned char* a1 = reinterpret_cast<unsigned char*>(S.a2);
     uint32_t phase = 0;
@@ -489,7 +491,8 @@ void lmac_set_attributes() {
 }
 
 void launch_walk_lmac_round(const NodeArrays& T, Counters* C, const int* leaf_list, const WalkParams& wp,
-                            const ListBuffers& LB, const LmacRounds& R, int round, int sm_count, cudaStream_t s) {
+                            const ListBuffers& LB, const LmacRounds& rounds, int round, int sm_count, cudaStream_t s) {
+    const LmacRounds R = round_pools(rounds, round);
     // persistent warps: one wave of resident CTAs (the global-stack variant
     // has one stack per warp of LB)
     if (wp.global_stack) {
@@ -498,12 +501,13 @@ void launch_walk_lmac_round(const NodeArrays& T, Counters* C, const int* leaf_li
     } else if (wp.smem_stack == 1024) {
         walk_lmac_round_kernel<1024, 8><<<sm_count * 8, kLwThreads, 0, s>>>(T, C, leaf_list, wp, LB, R, round);
     } else {
-        walk_lmac_round_kernel<2048, 6><<<sm_count * 6, kLwThreads, 0, s>>>(T, C, leaf_list, wp, LB, R, round);
+        walk_lmac_round_kernel<2048, 7><<<sm_count * 7, kLwThreads, 0, s>>>(T, C, leaf_list, wp, LB, R, round);
     }
 }
 
-void launch_lmac_infer(const NodeArrays& T, Counters* C, const WalkParams& wp, const LmacRounds& R, int round,
+void launch_lmac_infer(const NodeArrays& T, Counters* C, const WalkParams& wp, const LmacRounds& rounds, int round,
                        const LmacDev* model, int sm_count, cudaStream_t s) {
+    const LmacRounds R = round_pools(rounds, round);
     const size_t smem = tc_smem_bytes();
     // 64 tensor-memory columns per CTA: up to 8 CTAs per SM.
     lmac_infer_kernel<<<sm_count * 7, kLwThreads, smem, s>>>(T, C, wp, R, round, model);
