@@ -227,9 +227,8 @@ void enqueue_eval(ngrav_gpu_ctx* ctx, bool bbox_ready, bool kick, float hdt) {
     ctx->sort_passes = passes;
     launch_permute(P, ctx->SB.vals, n, split, s);
     // root, keys, 3 per sort pass (histogram, digit scans, scatter), permute,
-    // tree init, the levels, leaf list (mark, 3 scan kernels, compact), leaf
-    // moments, the internal-moment levels, walk
-    ctx->launches += 2 + (n > 1 ? 3 * passes : 0) + 1 + 1 + levels + 5 + 1 + levels + 1;
+    // tree init, the levels, leaf list (mark, 3 scan kernels, compact), walk
+    ctx->launches += 2 + (n > 1 ? 3 * passes : 0) + 1 + 1 + levels + 5 + 1;
     std::swap(P.pos, P.pos2);
     std::swap(P.plo, P.plo2);
     std::swap(P.vel, P.vel2);
@@ -242,8 +241,9 @@ void enqueue_eval(ngrav_gpu_ctx* ctx, bool bbox_ready, bool kick, float hdt) {
                        s);
     launch_leaf_list(ctx->T, ctx->C, n, ctx->leaf_at, ctx->flags, ctx->scanbuf, ctx->leaf_list, ctx->SB, s);
     rec(ctx, 3);
-    launch_moments(ctx->T, ctx->C, P, ctx->leaf_list, ctx->LB, n, (int)std::min<long long>(n, ctx->T.cap), split,
-                   ctx->opts.quadrupole != 0, levels, s);
+    ctx->launches += launch_moments(ctx->T, ctx->C, P, ctx->leaf_list, ctx->LB, n,
+                                    (int)std::min<long long>(n, ctx->T.cap), ctx->opts.leaf_capacity, split,
+                                    ctx->opts.quadrupole != 0, levels, s);
     rec(ctx, 4);
     WalkParams wp = walk_params(ctx, kick, hdt);
     const void* model = nullptr;

@@ -289,8 +289,9 @@ void launch_tree_levels(NodeArrays& T, Counters* C, const unsigned long long* ke
 void launch_leaf_list(NodeArrays& T, Counters* C, long long n, int* leaf_at, unsigned* flags, unsigned* scan_out,
                       int* leaf_list, SortBuffers& sb, cudaStream_t s);
 // Leaf and internal moments; also the evaluation's pass list (LB.passes).
-void launch_moments(NodeArrays& T, Counters* C, const Particles& P, const int* leaf_list, const ListBuffers& LB,
-                    long long n, int max_leaves, bool split, bool quadrupole, int levels, cudaStream_t s);
+// Returns the number of launches.
+int launch_moments(NodeArrays& T, Counters* C, const Particles& P, const int* leaf_list, const ListBuffers& LB,
+                   long long n, int max_leaves, int leaf_cap, bool split, bool quadrupole, int levels, cudaStream_t s);
 void launch_walk(const NodeArrays& T, Counters* C, const int* leaf_list, const WalkParams& wp,
                  const ListBuffers& LB, cudaStream_t s);
 void launch_eval(const NodeArrays& T, Counters* C, const Particles& P, const int* leaf_list, const WalkParams& wp,

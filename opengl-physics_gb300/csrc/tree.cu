@@ -16,6 +16,9 @@
 // per-node arrival counters so each parent is finished by the last child to
 // arrive.
 #include "engine.cuh"
+#include "walk_common.cuh"
+
+#include <algorithm>
 
 namespace ngrav {
 
@@ -280,13 +283,23 @@ __device__ __forceinline__ void write_walk_record(NodeArrays& T, int node, doubl
 // members of |a| from `acc` (the accelerations carried into this tree order;
 // zero before the first evaluation) that the learned opening test reads.
 //
-// GB300's FP64 pipe runs at 1/32 of the FP32 rate, so the per-particle work
+// GB300's FP64 pipe runs at 1/64 of the FP32 rate, so the per-particle work
 // is FP32: each member's offset from the leaf centre is a double-float pair
 // (error-free differences of the double-float position and centre), mass
 // and first moment are summed as double-float pairs with exact products,
 // and only the per-leaf results are FP64.  maxRadius keeps the reference's
 // FP64 value: the members within FP32 rounding of the FP32 maximum distance
 // are re-measured in FP64 (Tree.cpp:188-201).
+//
+// A warp takes `lpw` (4 to 32) consecutive leaves, and the FP64 steps run with a
+// lane per leaf, as one FP64 instruction occupies the pipe for 16 cycles however
+// few of its lanes are wanted.  Only the farthest member is re-measured, unless
+// a runner-up is within rounding of it: a re-measurement inside the member loop
+// stopped a warp in almost every iteration for one leaf or another.  Members are
+// read S lanes to a leaf: eight while there are few leaves, where the latency
+// of a leaf counts, one where there are many, which spares the reductions.
+// Before and now: 297 k leaves (4 Mi bodies) 278 and 156 us, 462 leaves (2,048
+// bodies) 27 and 13 us; eight lanes throughout took 185 us at 297 k leaves.
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
     s = a + b;
     const float bb = s - a;
@@ -315,41 +328,106 @@ __device__ __forceinline__ void df_add_prod(float& Sh, float& Sl, float m, float
     fast_two_sum(t, Sl + (e + pe), Sh, Sl);
 }
 
-__global__ void __launch_bounds__(128) moments_kernel(NodeArrays T, Counters* C, const float4* __restrict__ pos,
-                                                      const float4* __restrict__ plo, float4* __restrict__ src,
-                                                      const float4* __restrict__ acc,
-                                                      const int* __restrict__ leaf_list, int2* __restrict__ passes,
-                                                      int split, int quadrupole) {
-    const int nleaves = C->nleaves;
+// (ah, al) += (bh, bl)
+__device__ __forceinline__ void df_add(float& ah, float& al, float bh, float bl) {
+    float t, e;
+    two_sum(ah, bh, t, e);
+    fast_two_sum(t, al + (bl + e), ah, al);
+}
+
+__device__ __forceinline__ void df_add_xor(float& h, float& l, int o) {
+    const float oh = __shfl_xor_sync(0xffffffffu, h, o), ol = __shfl_xor_sync(0xffffffffu, l, o);
+    df_add(h, l, oh, ol);
+}
+
+// v of the leaf's lane, for the S lanes that work on leaf 32 / S * r + lane / S
+// (and back: the value that those lanes hold, kept by the leaf's lane).
+template <int S, typename V>
+__device__ __forceinline__ V to_members(V v, int r, int lane) {
+    return S == 1 ? v : __shfl_sync(0xffffffffu, v, 32 / S * r + lane / S);
+}
+
+template <int S, typename V>
+__device__ __forceinline__ void to_leaf(V& keep, V v, int r, int lane) {
+    if (S == 1) {
+        keep = v;
+    } else {
+        const V x = __shfl_sync(0xffffffffu, v, lane % (32 / S) * S);
+        if (lane / (32 / S) == r) keep = x;
+    }
+}
+
+constexpr int kMomFew = 16384, kMomWarps = 4;
+
+template <int S>
+__device__ __forceinline__ void leaf_moments(NodeArrays& T, Counters* C, const float4* __restrict__ pos,
+                                             const float4* __restrict__ plo, float4* __restrict__ src,
+                                             const float4* __restrict__ acc, const int* __restrict__ leaf_list,
+                                             int2* __restrict__ passes, int split, int quadrupole, int nleaves,
+                                             int lpw) {
     const int pass = pass_targets(nleaves);
     const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int li = blockIdx.x * blockDim.x + threadIdx.x; li < nleaves; li += gridDim.x * blockDim.x) {
-        const int leaf = leaf_list[li];
-        const int s = T.start[leaf], cnt = T.count[leaf];
-        if (cnt > pass) {
-            const int more = (cnt - 1) / pass;
-            const int at = atomicAdd(&C->extra_passes, more);
+    const int lane = threadIdx.x & 31, sub = lane % S;
+    const int nwarps = gridDim.x * kMomWarps;
+    for (long long first = (long long)(blockIdx.x * kMomWarps + (threadIdx.x >> 5)) * lpw; first < nleaves;
+         first += (long long)nwarps * lpw) {
+        // lane = leaf: the leaf's range and centre
+        const int li = (int)first + lane;
+        const bool has = lane < lpw && li < nleaves;
+        const int leaf = has ? leaf_list[li] : 0;
+        const int s = has ? T.start[leaf] : 0, cnt = has ? T.count[leaf] : 0;
+        const int more = cnt > pass ? (cnt - 1) / pass : 0;
+        int all_more;
+        const int before = warp_excl_scan(more, lane, all_more);
+        if (all_more > 0) {  // one atomic for the warp's leaves
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&C->extra_passes, all_more);
+            at = __shfl_sync(0xffffffffu, at, 0) + before;
             for (int p = 0; p < more; ++p) passes[at + p] = make_int2(li, p + 1);
         }
-        const double ccx = T.cx[leaf], ccy = T.cy[leaf], ccz = T.cz[leaf];
+        const double ccx = has ? T.cx[leaf] : 0.0, ccy = has ? T.cy[leaf] : 0.0, ccz = has ? T.cz[leaf] : 0.0;
+        const float half = has ? (float)T.half[leaf] : 0.f;
         const float chx = (float)ccx, chy = (float)ccy, chz = (float)ccz;
         const float clx = (float)(ccx - (double)chx), cly = (float)(ccy - (double)chy),
                     clz = (float)(ccz - (double)chz);
         // pass 1: mass and first moment about the leaf centre
         float Mh = 0.f, Ml = 0.f, Xh = 0.f, Xl = 0.f, Yh = 0.f, Yl = 0.f, Zh = 0.f, Zl = 0.f;
-        for (int j = s; j < s + cnt; ++j) {
-            const float4 p = pos[j];
-            const float4 q = plo ? plo[j] : zero4;
-            float ox, oxl, oy, oyl, oz, ozl;
-            df_offset(p.x, q.x, chx, clx, ox, oxl);
-            df_offset(p.y, q.y, chy, cly, oy, oyl);
-            df_offset(p.z, q.z, chz, clz, oz, ozl);
-            float t, e;
-            two_sum(Mh, p.w, t, e);
-            fast_two_sum(t, Ml + e, Mh, Ml);
-            df_add_prod(Xh, Xl, p.w, ox, oxl);
-            df_add_prod(Yh, Yl, p.w, oy, oyl);
-            df_add_prod(Zh, Zl, p.w, oz, ozl);
+        for (int r = 0; 32 / S * r < lpw; ++r) {
+            const int ms = to_members<S>(s, r, lane), mc = to_members<S>(cnt, r, lane);
+            const float hx = to_members<S>(chx, r, lane), hy = to_members<S>(chy, r, lane),
+                        hz = to_members<S>(chz, r, lane);
+            const float lx = to_members<S>(clx, r, lane), ly = to_members<S>(cly, r, lane),
+                        lz = to_members<S>(clz, r, lane);
+            float mh = 0.f, ml = 0.f, xh = 0.f, xl = 0.f, yh = 0.f, yl = 0.f, zh = 0.f, zl = 0.f;
+#pragma unroll 2
+            for (int j = sub; j < mc; j += S) {
+                const float4 p = pos[ms + j];
+                const float4 q = plo ? plo[ms + j] : zero4;
+                float ox, oxl, oy, oyl, oz, ozl;
+                df_offset(p.x, q.x, hx, lx, ox, oxl);
+                df_offset(p.y, q.y, hy, ly, oy, oyl);
+                df_offset(p.z, q.z, hz, lz, oz, ozl);
+                df_add(mh, ml, p.w, 0.f);
+                df_add_prod(xh, xl, p.w, ox, oxl);
+                df_add_prod(yh, yl, p.w, oy, oyl);
+                df_add_prod(zh, zl, p.w, oz, ozl);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int o = S / 2; o > 0; o >>= 1) {
+                df_add_xor(mh, ml, o);
+                df_add_xor(xh, xl, o);
+                df_add_xor(yh, yl, o);
+                df_add_xor(zh, zl, o);
+            }
+            to_leaf<S>(Mh, mh, r, lane);
+            to_leaf<S>(Ml, ml, r, lane);
+            to_leaf<S>(Xh, xh, r, lane);
+            to_leaf<S>(Xl, xl, r, lane);
+            to_leaf<S>(Yh, yh, r, lane);
+            to_leaf<S>(Yl, yl, r, lane);
+            to_leaf<S>(Zh, zh, r, lane);
+            to_leaf<S>(Zl, zl, r, lane);
         }
         const double M = (double)Mh + (double)Ml;
         double ocx = 0.0, ocy = 0.0, ocz = 0.0;  // COM - centre
@@ -363,66 +441,162 @@ __global__ void __launch_bounds__(128) moments_kernel(NodeArrays T, Counters* C,
         const float ohx = (float)ocx, ohy = (float)ocy, ohz = (float)ocz;
         const float olx = (float)(ocx - (double)ohx), oly = (float)(ocy - (double)ohy),
                     olz = (float)(ocz - (double)ohz);
-        // pass 2: FP32 distances from the COM, quadrupole, amin, walk sources
-        float maxf = 0.f;
-        float q0 = 0.f, q1 = 0.f, q2 = 0.f, q3 = 0.f, q4 = 0.f;
-        float amin2 = 3.0e38f;
-        for (int j = s; j < s + cnt; ++j) {
-            const float4 p = pos[j];
-            const float4 a = acc[j];
-            amin2 = fminf(amin2, a.x * a.x + a.y * a.y + a.z * a.z);
-            const float4 l = plo ? plo[j] : zero4;
-            float ox, oxl, oy, oyl, oz, ozl;
-            df_offset(p.x, l.x, chx, clx, ox, oxl);
-            df_offset(p.y, l.y, chy, cly, oy, oyl);
-            df_offset(p.z, l.z, chz, clz, oz, ozl);
-            const float fx = (ox - ohx) + (oxl - olx), fy = (oy - ohy) + (oyl - oly), fz = (oz - ohz) + (ozl - olz);
-            const float d2 = fmaf(fx, fx, fmaf(fy, fy, fz * fz));
-            maxf = fmaxf(maxf, d2);
-            if (quadrupole && cnt > 1) {
-                const float m = p.w;
-                q0 += m * (3.f * fx * fx - d2);
-                q1 += m * (3.f * fy * fy - d2);
-                q2 += m * 3.f * fx * fy;
-                q3 += m * 3.f * fx * fz;
-                q4 += m * 3.f * fy * fz;
+        // pass 2: FP32 distances from the COM, quadrupole, amin, walk sources,
+        // the farthest member and the runner-up's distance
+        float Q0 = 0.f, Q1 = 0.f, Q2 = 0.f, Q3 = 0.f, Q4 = 0.f, A2 = 0.f, Cut = 0.f;
+        int Far = -1;
+        bool several = false;
+        for (int r = 0; 32 / S * r < lpw; ++r) {
+            const int ms = to_members<S>(s, r, lane), mc = to_members<S>(cnt, r, lane);
+            const float hx = to_members<S>(chx, r, lane), hy = to_members<S>(chy, r, lane),
+                        hz = to_members<S>(chz, r, lane);
+            const float lx = to_members<S>(clx, r, lane), ly = to_members<S>(cly, r, lane),
+                        lz = to_members<S>(clz, r, lane);
+            const float ux = to_members<S>(ohx, r, lane), uy = to_members<S>(ohy, r, lane),
+                        uz = to_members<S>(ohz, r, lane);
+            const float vx = to_members<S>(olx, r, lane), vy = to_members<S>(oly, r, lane),
+                        vz = to_members<S>(olz, r, lane);
+            float maxf = -1.f, second = -1.f, amin2 = 3.0e38f;
+            int at = -1;
+            float q0 = 0.f, q1 = 0.f, q2 = 0.f, q3 = 0.f, q4 = 0.f;
+#pragma unroll 2
+            for (int j = sub; j < mc; j += S) {
+                const float4 p = pos[ms + j];
+                const float4 a = acc[ms + j];
+                const float4 l = plo ? plo[ms + j] : zero4;
+                amin2 = fminf(amin2, a.x * a.x + a.y * a.y + a.z * a.z);
+                float ox, oxl, oy, oyl, oz, ozl;
+                df_offset(p.x, l.x, hx, lx, ox, oxl);
+                df_offset(p.y, l.y, hy, ly, oy, oyl);
+                df_offset(p.z, l.z, hz, lz, oz, ozl);
+                const float fx = (ox - ux) + (oxl - vx), fy = (oy - uy) + (oyl - vy), fz = (oz - uz) + (ozl - vz);
+                const float d2 = fmaf(fx, fx, fmaf(fy, fy, fz * fz));
+                second = fmaxf(second, fminf(maxf, d2));
+                at = d2 > maxf ? j : at;
+                maxf = fmaxf(maxf, d2);
+                if (quadrupole && mc > 1) {
+                    const float m = p.w;
+                    q0 += m * (3.f * fx * fx - d2);
+                    q1 += m * (3.f * fy * fy - d2);
+                    q2 += m * 3.f * fx * fy;
+                    q3 += m * 3.f * fx * fz;
+                    q4 += m * 3.f * fy * fz;
+                }
+                src[ms + j] = split ? make_float4(ox + oxl, oy + oyl, oz + ozl, p.w) : p;
             }
-            src[j] = split ? make_float4(ox + oxl, oy + oyl, oz + ozl, p.w) : p;
+            __syncwarp();
+#pragma unroll
+            for (int o = S / 2; o > 0; o >>= 1) {
+                q0 += __shfl_xor_sync(0xffffffffu, q0, o);
+                q1 += __shfl_xor_sync(0xffffffffu, q1, o);
+                q2 += __shfl_xor_sync(0xffffffffu, q2, o);
+                q3 += __shfl_xor_sync(0xffffffffu, q3, o);
+                q4 += __shfl_xor_sync(0xffffffffu, q4, o);
+                amin2 = fminf(amin2, __shfl_xor_sync(0xffffffffu, amin2, o));
+                const float m2 = __shfl_xor_sync(0xffffffffu, maxf, o), s2 = __shfl_xor_sync(0xffffffffu, second, o);
+                const int at2 = __shfl_xor_sync(0xffffffffu, at, o);
+                second = fmaxf(fmaxf(second, s2), fminf(maxf, m2));
+                at = m2 > maxf || (m2 == maxf && at2 > at) ? at2 : at;
+                maxf = fmaxf(maxf, m2);
+            }
+            const float rcut = sqrtf(fmaxf(maxf, 0.f)) * (1.f - 4e-6f) - 2e-6f * to_members<S>(half, r, lane);
+            const float cut = rcut > 0.f ? rcut * rcut : -0.5f;
+            several |= second >= cut;
+            to_leaf<S>(Q0, q0, r, lane);
+            to_leaf<S>(Q1, q1, r, lane);
+            to_leaf<S>(Q2, q2, r, lane);
+            to_leaf<S>(Q3, q3, r, lane);
+            to_leaf<S>(Q4, q4, r, lane);
+            to_leaf<S>(A2, amin2, r, lane);
+            to_leaf<S>(Cut, cut, r, lane);
+            to_leaf<S>(Far, at, r, lane);
         }
         // pass 3: the FP64 maximum over the members that can hold it.  An FP32
         // distance is within a few ulps of the leaf's half size of the FP64
-        // one, so no member farther than the cut can be missed.
+        // one, so no member farther than the cut can be missed.  That is the
+        // farthest alone, unless a leaf of this warp has a runner-up past the
+        // cut: then all members are tested again, and the ones past it go to
+        // the leaf's lane as a mask per 64.
         double maxr2 = 0.0;
-        const float rcut = sqrtf(maxf) * (1.f - 4e-6f) - 2e-6f * (float)T.half[leaf];
-        const float cut = rcut > 0.f ? rcut * rcut : -1.f;
-        for (int j = s; j < s + cnt; ++j) {
+        auto measure = [&](int j) {
             const float4 p = pos[j];
             const float4 l = plo ? plo[j] : zero4;
-            float ox, oxl, oy, oyl, oz, ozl;
-            df_offset(p.x, l.x, chx, clx, ox, oxl);
-            df_offset(p.y, l.y, chy, cly, oy, oyl);
-            df_offset(p.z, l.z, chz, clz, oz, ozl);
-            const float fx = (ox - ohx) + (oxl - olx), fy = (oy - ohy) + (oyl - oly), fz = (oz - ohz) + (ozl - olz);
-            if (fmaf(fx, fx, fmaf(fy, fy, fz * fz)) >= cut) {
-                const double x = (double)p.x + (double)l.x, y = (double)p.y + (double)l.y,
-                             z = (double)p.z + (double)l.z;
-                const double dx = x - cx, dy = y - cy, dz = z - cz;
-                maxr2 = fmax(maxr2, dx * dx + dy * dy + dz * dz);
+            const double x = (double)p.x + (double)l.x, y = (double)p.y + (double)l.y, z = (double)p.z + (double)l.z;
+            const double dx = x - cx, dy = y - cy, dz = z - cz;
+            maxr2 = fmax(maxr2, dx * dx + dy * dy + dz * dz);
+        };
+        if (!__any_sync(0xffffffffu, several)) {
+            if (has && Far >= 0) measure(s + Far);
+        } else {
+            int most = cnt;
+            for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+            for (int m0 = 0; m0 < most; m0 += 64) {
+                unsigned long long cand = 0;
+                for (int r = 0; 32 / S * r < lpw; ++r) {
+                    const int ms = to_members<S>(s, r, lane), mc = min(to_members<S>(cnt, r, lane), m0 + 64);
+                    const float hx = to_members<S>(chx, r, lane), hy = to_members<S>(chy, r, lane),
+                                hz = to_members<S>(chz, r, lane);
+                    const float lx = to_members<S>(clx, r, lane), ly = to_members<S>(cly, r, lane),
+                                lz = to_members<S>(clz, r, lane);
+                    const float ux = to_members<S>(ohx, r, lane), uy = to_members<S>(ohy, r, lane),
+                                uz = to_members<S>(ohz, r, lane);
+                    const float vx = to_members<S>(olx, r, lane), vy = to_members<S>(oly, r, lane),
+                                vz = to_members<S>(olz, r, lane);
+                    const float cut = to_members<S>(Cut, r, lane);
+                    unsigned long long mine = 0;  // of this lane's members
+                    for (int j = m0 + sub; j < mc; j += S) {
+                        const float4 p = pos[ms + j];
+                        const float4 l = plo ? plo[ms + j] : zero4;
+                        float ox, oxl, oy, oyl, oz, ozl;
+                        df_offset(p.x, l.x, hx, lx, ox, oxl);
+                        df_offset(p.y, l.y, hy, ly, oy, oyl);
+                        df_offset(p.z, l.z, hz, lz, oz, ozl);
+                        const float fx = (ox - ux) + (oxl - vx), fy = (oy - uy) + (oyl - vy),
+                                    fz = (oz - uz) + (ozl - vz);
+                        if (fmaf(fx, fx, fmaf(fy, fy, fz * fz)) >= cut) mine |= 1ull << (j - m0);
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int o = S / 2; o > 0; o >>= 1) mine |= __shfl_xor_sync(0xffffffffu, mine, o);
+                    to_leaf<S>(cand, mine, r, lane);
+                }
+                while (cand) {
+                    measure(s + m0 + __ffsll((long long)cand) - 1);
+                    cand &= cand - 1;
+                }
+                __syncwarp();
             }
         }
-        const double maxr = sqrt(maxr2);
-        const double Q[5] = {q0, q1, q2, q3, q4};
-        T.mass[leaf] = M;
-        T.comx[leaf] = cx;
-        T.comy[leaf] = cy;
-        T.comz[leaf] = cz;
-        T.maxr[leaf] = maxr;
-        T.amin[leaf] = cnt > 0 ? sqrtf(amin2) : 0.f;
-        for (int k = 0; k < 5; ++k) T.quad[5 * leaf + k] = Q[k];
-        const int level = T.level[leaf];
-        write_walk_record(T, leaf, M, cx, cy, cz, Q, maxr, true, s, cnt, level);
-        T.chi[leaf] = make_float4(chx, chy, chz, __int_as_float(s));
-        T.clo[leaf] = make_float4(clx, cly, clz, __int_as_float(cnt));
+        if (has) {
+            const double maxr = sqrt(maxr2);
+            const double Q[5] = {Q0, Q1, Q2, Q3, Q4};
+            T.mass[leaf] = M;
+            T.comx[leaf] = cx;
+            T.comy[leaf] = cy;
+            T.comz[leaf] = cz;
+            T.maxr[leaf] = maxr;
+            T.amin[leaf] = cnt > 0 ? sqrtf(A2) : 0.f;
+            for (int k = 0; k < 5; ++k) T.quad[5 * leaf + k] = Q[k];
+            const int level = T.level[leaf];
+            write_walk_record(T, leaf, M, cx, cy, cz, Q, maxr, true, s, cnt, level);
+            T.chi[leaf] = make_float4(chx, chy, chz, __int_as_float(s));
+            T.clo[leaf] = make_float4(clx, cly, clz, __int_as_float(cnt));
+        }
+        __syncwarp();
+    }
+}
+
+__global__ void __launch_bounds__(32 * kMomWarps, 6)
+    moments_kernel(NodeArrays T, Counters* C, const float4* __restrict__ pos, const float4* __restrict__ plo,
+                   float4* __restrict__ src, const float4* __restrict__ acc, const int* __restrict__ leaf_list,
+                   int2* __restrict__ passes, int split, int quadrupole) {
+    const int nleaves = C->nleaves;
+    if (nleaves <= kMomFew) {
+        // as few leaves per warp as four while an SM has few warps
+        const int lpw = nleaves <= 4 * 152 * kMomWarps ? 4 : nleaves <= 8 * 152 * kMomWarps ? 8 : 16;
+        leaf_moments<8>(T, C, pos, plo, src, acc, leaf_list, passes, split, quadrupole, nleaves, lpw);
+    } else {
+        leaf_moments<1>(T, C, pos, plo, src, acc, leaf_list, passes, split, quadrupole, nleaves, 32);
     }
 }
 
@@ -437,11 +611,13 @@ __global__ void __launch_bounds__(128) moments_kernel(NodeArrays T, Counters* C,
 // the children within rounding of the FP32 maximum re-measured in FP64.  The
 // geometric opening test reads maxRadius of leaves only; the learned one
 // reads it for every node.
-__global__ void __launch_bounds__(256) internal_moments_kernel(NodeArrays T, const Counters* __restrict__ C, int l,
-                                                              int quadrupole) {
-    const int begin = C->level_begin[l];
-    const int end = C->level_begin[l + 1];
-    for (int node = begin + blockIdx.x * blockDim.x + threadIdx.x; node < end; node += gridDim.x * blockDim.x) {
+//
+// The re-measured children wait in a mask, so that a warp runs the FP64 square
+// root once or twice and not once for each of the eight places (4 Mi bodies, 16
+// levels: 280 and 166 us).
+__device__ __forceinline__ void internal_moments(NodeArrays& T, int begin, int end, int tid, int nthreads, int l,
+                                                 int quadrupole) {
+    for (int node = begin + tid; node < end; node += nthreads) {
         const int fc = T.first_child[node];
         if (fc < 0) continue;
         const int nch = T.nchild[node];
@@ -500,14 +676,18 @@ __global__ void __launch_bounds__(256) internal_moments_kernel(NodeArrays T, con
             best = fmaxf(best, cand[k]);
         }
         double mr = 0.0;
+        unsigned past = 0;
         if (PM > 0.0) {
             const float cut = best * (1.f - 1e-5f) - 1e-30f;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                if (k >= nch || cand[k] < cut) continue;
-                const double dx = cxs[k] - pcx, dy = cys[k] - pcy, dz = czs[k] - pcz;
-                mr = fmax(mr, T.maxr[fc + k] + sqrt(dx * dx + dy * dy + dz * dz));
-            }
+            for (int k = 0; k < 8; ++k)
+                if (k < nch && !(cand[k] < cut)) past |= 1u << k;
+        }
+        while (past) {
+            const int c = fc + __ffs((int)past) - 1;
+            past &= past - 1;
+            const double dx = T.comx[c] - pcx, dy = T.comy[c] - pcy, dz = T.comz[c] - pcz;
+            mr = fmax(mr, T.maxr[c] + sqrt(dx * dx + dy * dy + dz * dz));
         }
         const double PQ[5] = {q0, q1, q2, q3, q4};
         T.mass[node] = PM;
@@ -520,18 +700,54 @@ __global__ void __launch_bounds__(256) internal_moments_kernel(NodeArrays T, con
     }
 }
 
-void launch_moments(NodeArrays& T, Counters* C, const Particles& P, const int* leaf_list, const ListBuffers& LB,
-                    long long n, int max_leaves, bool split, bool quadrupole, int levels, cudaStream_t s) {
-    long long blocks = ((long long)max_leaves + 127) / 128;
+constexpr int kIntThreads = 64;
+
+__global__ void __launch_bounds__(kIntThreads) internal_moments_kernel(NodeArrays T, const Counters* __restrict__ C,
+                                                                      int l, int quadrupole) {
+    internal_moments(T, C->level_begin[l], C->level_begin[l + 1], blockIdx.x * blockDim.x + threadIdx.x,
+                     gridDim.x * blockDim.x, l, quadrupole);
+}
+
+// Levels `levels` - 1 down to 0 in one launch: one cluster, its barrier between
+// two levels (arrive.release / wait.acquire at cluster scope orders the
+// records that its CTAs exchange through global memory).
+constexpr int kTopCtas = 8, kTopThreads = 256;
+
+__global__ void __cluster_dims__(kTopCtas, 1, 1) __launch_bounds__(kTopThreads)
+    top_moments_kernel(NodeArrays T, const Counters* __restrict__ C, int levels, int quadrupole) {
+    for (int l = levels - 1; l >= 0; --l) {
+        // neighbouring nodes go to different SMs by whole warps
+        const int tid = ((threadIdx.x >> 5) * kTopCtas + blockIdx.x) * 32 + (threadIdx.x & 31);
+        internal_moments(T, C->level_begin[l], C->level_begin[l + 1], tid, kTopCtas * kTopThreads, l, quadrupole);
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+}
+
+// The top levels, of at most 8^3 nodes each, go to the cluster, and so do all
+// levels of a tree of few nodes: a level is a chain of latencies, some 6 us in the
+// cluster (2,048 bodies, 9 levels: 56 us) and 10 in a launch of its own (89 us), but
+// a cluster has 8 of the 152 SMs' FP64 pipes.  All of the moments with every level
+// in the cluster, and with the top four: 63 and 78 us at 2,048 bodies, 86 and 107
+// at 20,011 (leaves of 8), 143 and 131 at 131,071 (leaves of 16).
+constexpr int kTopLevels = 4;
+constexpr long long kTopTree = 4096;  // bodies per leaf_capacity of a tree of few nodes
+
+int launch_moments(NodeArrays& T, Counters* C, const Particles& P, const int* leaf_list, const ListBuffers& LB,
+                    long long n, int max_leaves, int leaf_cap, bool split, bool quadrupole, int levels,
+                    cudaStream_t s) {
+    long long blocks = ((long long)max_leaves + 4 * kMomWarps - 1) / (4 * kMomWarps);
     if (blocks > 152 * 16) blocks = 152 * 16;
     if (blocks < 1) blocks = 1;
-    moments_kernel<<<(unsigned)blocks, 128, 0, s>>>(T, C, P.pos, split ? P.plo : nullptr, P.src, P.acc, leaf_list,
-                                                    LB.passes, split ? 1 : 0, quadrupole ? 1 : 0);
-    long long b2 = ((long long)T.cap / 4 + 255) / 256;
-    if (b2 > 152 * 4) b2 = 152 * 4;
+    moments_kernel<<<(unsigned)blocks, 32 * kMomWarps, 0, s>>>(T, C, P.pos, split ? P.plo : nullptr, P.src, P.acc,
+                                                               leaf_list, LB.passes, split ? 1 : 0, quadrupole ? 1 : 0);
+    const int top = n <= kTopTree * leaf_cap ? levels : std::min(levels, kTopLevels);
+    long long b2 = ((long long)T.cap / 4 + kIntThreads - 1) / kIntThreads;
+    if (b2 > 152 * 8) b2 = 152 * 8;
     if (b2 < 1) b2 = 1;
-    for (int l = levels - 1; l >= 0; --l)
-        internal_moments_kernel<<<(unsigned)b2, 256, 0, s>>>(T, C, l, quadrupole ? 1 : 0);
+    for (int l = levels - 1; l >= top; --l)
+        internal_moments_kernel<<<(unsigned)b2, kIntThreads, 0, s>>>(T, C, l, quadrupole ? 1 : 0);
+    top_moments_kernel<<<kTopCtas, kTopThreads, 0, s>>>(T, C, top, quadrupole ? 1 : 0);
+    return 2 + levels - top;
 }
 
 void launch_reset_counters(Counters* C, cudaStream_t s) { reset_counters_kernel<<<1, 32, 0, s>>>(C); }
