@@ -58,17 +58,18 @@ void free_particles(ngrav_gpu_ctx* ctx) {
     dfree(P.pos2); dfree(P.plo2); dfree(P.vel2); dfree(P.vlo2); dfree(P.acc2); dfree(P.id2);
     P.cap = 0;
     SortBuffers& S = ctx->SB;
-    dfree(S.keys); dfree(S.keys_alt); dfree(S.vals); dfree(S.vals_alt); dfree(S.hist); dfree(S.scan_tmp);
+    dfree(S.keys); dfree(S.keys_alt); dfree(S.vals); dfree(S.vals_alt); dfree(S.hist);
     dfree(S.ktab);
     S.cap = 0;
-    dfree(ctx->leaf_at); dfree(ctx->flags); dfree(ctx->scanbuf); dfree(ctx->leaf_list);
+    TreeBuffers& B = ctx->TB;
+    dfree(B.runs); dfree(B.counts); dfree(B.leaf_list); dfree(B.leaf_before); dfree(B.leaf_start);
     dfree(ctx->stage); dfree(ctx->inv);
     ctx->cap_n = 0;
 }
 
 void free_nodes(ngrav_gpu_ctx* ctx) {
     NodeArrays& T = ctx->T;
-    dfree(T.start); dfree(T.count); dfree(T.first_child); dfree(T.parent); dfree(T.visit);
+    dfree(T.start); dfree(T.count); dfree(T.first_child); dfree(T.parent);
     dfree(T.nchild); dfree(T.level); dfree(T.cx); dfree(T.cy); dfree(T.cz); dfree(T.half); dfree(T.sysroot);
     dfree(T.mass); dfree(T.comx); dfree(T.comy); dfree(T.comz); dfree(T.maxr); dfree(T.quad); dfree(T.amin);
     dfree(T.wA); dfree(T.wB); dfree(T.wC); dfree(T.wD); dfree(T.chi); dfree(T.clo);
@@ -91,12 +92,11 @@ int alloc_particles(ngrav_gpu_ctx* ctx, long long n) {
     NG_CUDA(dalloc(S.vals_alt, c));
     S.hist_cap = radix_hist_size(c);
     NG_CUDA(dalloc(S.hist, S.hist_cap));
-    S.scan_tmp_cap = scan_tmp_size(std::max(S.hist_cap, c)) + 16;
-    NG_CUDA(dalloc(S.scan_tmp, S.scan_tmp_cap));
     NG_CUDA(dalloc(S.ktab, key_table_entries()));
     S.cap = c;
-    NG_CUDA(dalloc(ctx->leaf_at, c)); NG_CUDA(dalloc(ctx->flags, c)); NG_CUDA(dalloc(ctx->scanbuf, c));
-    NG_CUDA(dalloc(ctx->leaf_list, c)); NG_CUDA(dalloc(ctx->inv, c));
+    TreeBuffers& B = ctx->TB;
+    NG_CUDA(dalloc(B.runs, c)); NG_CUDA(dalloc(B.counts, tree_counts_size())); NG_CUDA(dalloc(B.leaf_list, c));
+    NG_CUDA(dalloc(B.leaf_before, c)); NG_CUDA(dalloc(B.leaf_start, c)); NG_CUDA(dalloc(ctx->inv, c));
     NG_CUDA(dalloc(ctx->stage, 7 * c));
     ctx->cap_n = c;
     return NGRAV_OK;
@@ -106,7 +106,7 @@ int alloc_nodes(ngrav_gpu_ctx* ctx, int cap) {
     free_nodes(ctx);
     NodeArrays& T = ctx->T;
     NG_CUDA(dalloc(T.start, cap)); NG_CUDA(dalloc(T.count, cap)); NG_CUDA(dalloc(T.first_child, cap));
-    NG_CUDA(dalloc(T.parent, cap)); NG_CUDA(dalloc(T.visit, cap)); NG_CUDA(dalloc(T.nchild, cap));
+    NG_CUDA(dalloc(T.parent, cap)); NG_CUDA(dalloc(T.nchild, cap));
     NG_CUDA(dalloc(T.level, cap)); NG_CUDA(dalloc(T.cx, cap)); NG_CUDA(dalloc(T.cy, cap)); NG_CUDA(dalloc(T.cz, cap));
     NG_CUDA(dalloc(T.half, cap)); NG_CUDA(dalloc(T.sysroot, cap));
     NG_CUDA(dalloc(T.mass, cap)); NG_CUDA(dalloc(T.comx, cap)); NG_CUDA(dalloc(T.comy, cap));
@@ -227,8 +227,8 @@ void enqueue_eval(ngrav_gpu_ctx* ctx, bool bbox_ready, bool kick, float hdt) {
     ctx->sort_passes = passes;
     launch_permute(P, ctx->SB.vals, n, split, s);
     // root, keys, 3 per sort pass (histogram, digit scans, scatter), permute,
-    // tree init, the levels, leaf list (mark, 3 scan kernels, compact), walk
-    ctx->launches += 2 + (n > 1 ? 3 * passes : 0) + 1 + 1 + levels + 5 + 1;
+    // walk
+    ctx->launches += 2 + (n > 1 ? 3 * passes : 0) + 1 + 1;
     std::swap(P.pos, P.pos2);
     std::swap(P.plo, P.plo2);
     std::swap(P.vel, P.vel2);
@@ -236,25 +236,24 @@ void enqueue_eval(ngrav_gpu_ctx* ctx, bool bbox_ready, bool kick, float hdt) {
     std::swap(P.acc, P.acc2);
     std::swap(P.id, P.id2);
     rec(ctx, 2);
-    launch_tree_init(ctx->T, ctx->C, n, ctx->opts.leaf_capacity, ctx->opts.max_depth, s);
-    launch_tree_levels(ctx->T, ctx->C, ctx->SB.keys, n, ctx->opts.leaf_capacity, ctx->opts.max_depth, ctx->F, levels,
-                       s);
-    launch_leaf_list(ctx->T, ctx->C, n, ctx->leaf_at, ctx->flags, ctx->scanbuf, ctx->leaf_list, ctx->SB, s);
+    const bool per_particle = ctx->block_on || ctx->opts.mac == NGRAV_MAC_RELATIVE;
+    ctx->launches += launch_tree(ctx->T, ctx->C, ctx->SB.keys, n, ctx->opts.leaf_capacity, ctx->opts.max_depth, ctx->F,
+                                 levels, ctx->TB, per_particle, s);
     rec(ctx, 3);
-    ctx->launches += launch_moments(ctx->T, ctx->C, P, ctx->leaf_list, ctx->LB, n,
+    ctx->launches += launch_moments(ctx->T, ctx->C, P, ctx->TB.leaf_list, ctx->LB, n,
                                     (int)std::min<long long>(n, ctx->T.cap), ctx->opts.leaf_capacity, split,
                                     ctx->opts.quadrupole != 0, levels, s);
     rec(ctx, 4);
     WalkParams wp = walk_params(ctx, kick, hdt);
     const void* model = nullptr;
-    if (ctx->block_on || ctx->opts.mac == NGRAV_MAC_RELATIVE) {
+    if (per_particle) {
         // per-particle walk: decisions, sums and the closing kick in one
         // kernel; block timesteps take the geometric test on their targets
         // (ComputeAccelBarnesHutTargets, Solvers.cpp:384-405)
         rec(ctx, 5);
-        launch_walk_pp(ctx->T, ctx->C, P, ctx->leaf_list, wp, ctx->block_on ? 0 : 1, ctx->alpha, nullptr,
-                       ctx->block_on ? ctx->block_args : nullptr, ctx->block_base, n, ctx->scanbuf, ctx->flags,
-                       ctx->LB.nwarps, s);
+        launch_walk_pp(ctx->T, ctx->C, P, ctx->TB.leaf_list, wp, ctx->block_on ? 0 : 1, ctx->alpha, nullptr,
+                       ctx->block_on ? ctx->block_args : nullptr, ctx->block_base, n, ctx->TB.leaf_before,
+                       ctx->TB.leaf_start, ctx->LB.nwarps, s);
         rec(ctx, 6);
         ctx->launches += 1;
         return;
@@ -262,9 +261,9 @@ void enqueue_eval(ngrav_gpu_ctx* ctx, bool bbox_ready, bool kick, float hdt) {
     if (lmac_walk_setup(ctx, wp, &model))
         lmac_launch_walk(ctx, wp, model);
     else
-        launch_walk(ctx->T, ctx->C, ctx->leaf_list, wp, ctx->LB, s);
+        launch_walk(ctx->T, ctx->C, ctx->TB.leaf_list, wp, ctx->LB, s);
     rec(ctx, 5);
-    launch_eval(ctx->T, ctx->C, P, ctx->leaf_list, wp, ctx->LB, ctx->eval_nwarps, s);
+    launch_eval(ctx->T, ctx->C, P, ctx->TB.leaf_list, wp, ctx->LB, ctx->eval_nwarps, s);
     rec(ctx, 6);
     ctx->launches += 1;  // the evaluation kernel
 }
@@ -447,10 +446,7 @@ std::vector<unsigned char> step_key(const ngrav_gpu_ctx* ctx, float hdt, float f
     put(&ctx->SB, sizeof(ctx->SB));
     put(&ctx->LB, sizeof(ctx->LB));
     put(&ctx->C, sizeof(ctx->C));
-    put(&ctx->leaf_at, sizeof(ctx->leaf_at));
-    put(&ctx->flags, sizeof(ctx->flags));
-    put(&ctx->scanbuf, sizeof(ctx->scanbuf));
-    put(&ctx->leaf_list, sizeof(ctx->leaf_list));
+    put(&ctx->TB, sizeof(ctx->TB));
     put(&ctx->n, sizeof(ctx->n));
     put(&ctx->opts, sizeof(ctx->opts));
     put(&ctx->walk_global_stack, sizeof(ctx->walk_global_stack));

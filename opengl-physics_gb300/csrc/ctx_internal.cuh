@@ -29,10 +29,7 @@ struct ngrav_gpu_ctx {
     NodeArrays T;
     Counters* C = nullptr;
     Counters hc{};
-    int* leaf_at = nullptr;
-    unsigned* flags = nullptr;
-    unsigned* scanbuf = nullptr;
-    int* leaf_list = nullptr;
+    TreeBuffers TB;
     ListBuffers LB;
     int eval_nwarps = 0;
     long long gi_cap = 0;

@@ -58,7 +58,7 @@ void launch_forest_potential(const Particles& P, bool split, const Forest& F, do
 // walk_pp.cu: the per-particle walk (relative MAC, target subsets), with the
 // force sums and the closing kick.
 // block = {sub, rmax}: block-timestep mode (nullptr: every particle).
-// before / starts: the scan and the flags of launch_leaf_list.
+// before / starts: TreeBuffers::leaf_before and leaf_start.
 void walk_pp_set_attributes();
 void launch_walk_pp(const NodeArrays& T, Counters* C, const Particles& P, const int* leaf_list, const WalkParams& wp,
                     int relative, double alpha, const unsigned char* targets, const int* block, double block_base,

@@ -111,13 +111,21 @@ struct ListBuffers {
     int nwarps = 0;                   // resident walking warps
 };
 
+// Scratch of the topology build, and the leaves it lists in key order.
+struct TreeBuffers {
+    unsigned short* runs = nullptr;   // per particle: the levels of the nodes that begin at it
+    int* counts = nullptr;            // nodes per level and leaves, per segment of the particles; their totals
+    int* leaf_list = nullptr;
+    unsigned* leaf_before = nullptr;  // per particle: the leaves that begin before it,
+    unsigned* leaf_start = nullptr;   // and whether one begins at it
+};
+
 struct NodeArrays {
     int cap = 0;
     int* start = nullptr;
     int* count = nullptr;
     int* first_child = nullptr;       // -1 for leaves
     int* parent = nullptr;
-    int* visit = nullptr;             // upward-pass arrival counters
     unsigned char* nchild = nullptr;
     unsigned char* level = nullptr;
     double* cx = nullptr;             // geometric centre (FP64 recurrence of the reference)
@@ -173,9 +181,7 @@ struct SortBuffers {
     unsigned* vals = nullptr;
     unsigned* vals_alt = nullptr;
     unsigned* hist = nullptr;         // kRsBins x blocks
-    unsigned* scan_tmp = nullptr;
     long long hist_cap = 0;
-    long long scan_tmp_cap = 0;
     long long* ktab = nullptr;        // centres of the top key levels, ordered images (key_table_entries())
 };
 
@@ -281,13 +287,14 @@ long long radix_hist_size(long long n);
 // Doubles of SortBuffers::ktab: the tabulated key centres of the three axes.
 long long key_table_entries();
 void launch_permute(const Particles& P, const unsigned* perm, long long n, bool split, cudaStream_t s);
-void launch_tree_init(NodeArrays& T, Counters* C, long long n, int leaf_cap, int max_depth, cudaStream_t s);
-// Builds levels 1 .. levels (keys sorted on their top `levels` digits); a node
-// at level `levels` that would still split sets kStSortDepth.
-void launch_tree_levels(NodeArrays& T, Counters* C, const unsigned long long* keys, long long n, int leaf_cap,
-                        int max_depth, const Forest& F, int levels, cudaStream_t s);
-void launch_leaf_list(NodeArrays& T, Counters* C, long long n, int* leaf_at, unsigned* flags, unsigned* scan_out,
-                      int* leaf_list, SortBuffers& sb, cudaStream_t s);
+// Builds the nodes down to level `levels` (keys sorted on their top `levels`
+// digits; a node there that would still split sets kStSortDepth) and the leaf
+// list; with leaf_scan also B.leaf_before and B.leaf_start.  Returns the number
+// of launches.
+int launch_tree(NodeArrays& T, Counters* C, const unsigned long long* keys, long long n, int leaf_cap, int max_depth,
+                const Forest& F, int levels, const TreeBuffers& B, bool leaf_scan, cudaStream_t s);
+// Entries of TreeBuffers::counts.
+long long tree_counts_size();
 // Leaf and internal moments; also the evaluation's pass list (LB.passes).
 // Returns the number of launches.
 int launch_moments(NodeArrays& T, Counters* C, const Particles& P, const int* leaf_list, const ListBuffers& LB,
@@ -299,7 +306,5 @@ void launch_eval(const NodeArrays& T, Counters* C, const Particles& P, const int
 void launch_kick_drift(const Particles& P, long long n, float hdt, float dt, bool split, Counters* C,
                        cudaStream_t s);
 void launch_scatter_accel(const Particles& P, long long n, double* ax, double* ay, double* az, cudaStream_t s);
-void device_exclusive_scan(const unsigned* in, unsigned* out, long long n, unsigned* tmp, cudaStream_t s);
-long long scan_tmp_size(long long n);
 
 }  // namespace ngrav

@@ -1,6 +1,6 @@
 // keys_sort.cu -- bounding box, 63-bit octant-path keys, stable LSD radix
-// sort of (key, slot) pairs, device-wide exclusive scan and the gather that
-// puts the particle state into key order.
+// sort of (key, slot) pairs and the gather that puts the particle state into
+// key order.
 //
 // Bit-exactness with the reference tree (projects/nbody_core/src/Tree.cpp):
 //  * the root cube is the FP64 bounding box of the positions, centre
@@ -407,16 +407,6 @@ int launch_keys(const float4* pos, const float4* plo, long long n, Counters* C, 
     return 1;
 }
 
-// ---------------------------------------------------------------------------
-// Device-wide exclusive scan of unsigned (reduce / scan partials / downsweep)
-// ---------------------------------------------------------------------------
-
-constexpr int kScanThreads = 512;
-constexpr int kScanItems = 8;
-constexpr int kScanTile = kScanThreads * kScanItems;
-
-long long scan_tmp_size(long long n) { return (n + kScanTile - 1) / kScanTile + 1; }
-
 // Block-wide exclusive scan of one value per thread; returns the block total.
 __device__ __forceinline__ unsigned block_exclusive_scan(unsigned v, unsigned* s_warp, unsigned& total) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -440,70 +430,6 @@ __device__ __forceinline__ unsigned block_exclusive_scan(unsigned v, unsigned* s
     const unsigned before = w > 0 ? s_warp[w - 1] : 0u;
     __syncthreads();
     return before + x - v;
-}
-
-__global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(const unsigned* __restrict__ in, long long n,
-                                                                   unsigned* __restrict__ partial) {
-    const long long base = blockIdx.x * (long long)kScanTile;
-    unsigned s = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        const long long i = base + k * kScanThreads + threadIdx.x;
-        if (i < n) s += in[i];
-    }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    __shared__ unsigned ws[kScanThreads / 32];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned t = 0;
-        for (int k = 0; k < kScanThreads / 32; ++k) t += ws[k];
-        partial[blockIdx.x] = t;
-    }
-}
-
-__global__ void __launch_bounds__(1024) scan_partials_kernel(unsigned* partial, int nb) {
-    __shared__ unsigned s_warp[32];
-    unsigned carry = 0;
-    for (int base = 0; base < nb; base += 1024) {
-        const int i = base + threadIdx.x;
-        const unsigned v = i < nb ? partial[i] : 0u;
-        unsigned total;
-        const unsigned ex = block_exclusive_scan(v, s_warp, total);
-        if (i < nb) partial[i] = carry + ex;
-        carry += total;
-    }
-}
-
-__global__ void __launch_bounds__(kScanThreads) scan_down_kernel(const unsigned* __restrict__ in, long long n,
-                                                                 const unsigned* __restrict__ partial,
-                                                                 unsigned* __restrict__ out) {
-    __shared__ unsigned s_warp[32];
-    const long long base = blockIdx.x * (long long)kScanTile + (long long)threadIdx.x * kScanItems;
-    unsigned v[kScanItems];
-    unsigned sum = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        const long long i = base + k;
-        v[k] = i < n ? in[i] : 0u;
-        sum += v[k];
-    }
-    unsigned total;
-    unsigned run = block_exclusive_scan(sum, s_warp, total) + partial[blockIdx.x];
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        const long long i = base + k;
-        if (i < n) out[i] = run;
-        run += v[k];
-    }
-}
-
-void device_exclusive_scan(const unsigned* in, unsigned* out, long long n, unsigned* tmp, cudaStream_t s) {
-    if (n <= 0) return;
-    const int nb = (int)((n + kScanTile - 1) / kScanTile);
-    scan_reduce_kernel<<<nb, kScanThreads, 0, s>>>(in, n, tmp);
-    scan_partials_kernel<<<1, 1024, 0, s>>>(tmp, nb);
-    scan_down_kernel<<<nb, kScanThreads, 0, s>>>(in, n, tmp, out);
 }
 
 // ---------------------------------------------------------------------------

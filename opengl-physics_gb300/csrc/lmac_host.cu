@@ -175,7 +175,7 @@ int collect_pairs(ngrav_gpu_ctx* ctx, float theta_rec, float rho_lo, float rho_h
     LmacState& L = *ctx->lm;
     cudaStream_t s = ctx->stream;
     NG_TRY(ensure_pairs(ctx, std::max(cap, 1)));
-    launch_lmac_amin(ctx->T, ctx->C, ctx->leaf_list, ctx->P.acc, std::min<long long>(ctx->n, ctx->T.cap), s);
+    launch_lmac_amin(ctx->T, ctx->C, ctx->TB.leaf_list, ctx->P.acc, std::min<long long>(ctx->n, ctx->T.cap), s);
     NG_CUDA(cudaMemsetAsync(L.dCnt, 0, 4 * sizeof(unsigned long long), s));
     NG_CUDA(cudaMemsetAsync(L.dWork, 0, sizeof(int), s));
     LmacRecordParams rp{};
@@ -192,7 +192,7 @@ int collect_pairs(ngrav_gpu_ctx* ctx, float theta_rec, float rho_lo, float rho_h
     rp.nkept = L.dCnt;
     rp.nband = L.dCnt + 1;
     rp.ndropped = L.dCnt + 2;
-    launch_lmac_record(ctx->T, ctx->C, ctx->leaf_list, rp, ctx->sm_count * 4, s);
+    launch_lmac_record(ctx->T, ctx->C, ctx->TB.leaf_list, rp, ctx->sm_count * 4, s);
     unsigned long long cnt[3];
     NG_CUDA(cudaMemcpyAsync(cnt, L.dCnt, sizeof(cnt), cudaMemcpyDeviceToHost, s));
     NG_CUDA(cudaStreamSynchronize(s));
@@ -355,7 +355,7 @@ void lmac_launch_walk(ngrav_gpu_ctx* ctx, const WalkParams& wp, const void* mode
     cudaStream_t s = ctx->stream;
     cudaMemsetAsync(L.R.ctr, 0, sizeof(int) * 4 * kLmMaxRounds, s);
     for (int r = 0; r < L.R.rounds; ++r) {
-        launch_walk_lmac_round(ctx->T, ctx->C, ctx->leaf_list, wp, ctx->LB, L.R, r, ctx->sm_count, s);
+        launch_walk_lmac_round(ctx->T, ctx->C, ctx->TB.leaf_list, wp, ctx->LB, L.R, r, ctx->sm_count, s);
         if (r + 1 < L.R.rounds)
             launch_lmac_infer(ctx->T, ctx->C, wp, L.R, r, static_cast<const LmacDev*>(model), ctx->sm_count, s);
     }

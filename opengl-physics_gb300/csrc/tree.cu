@@ -4,17 +4,13 @@
 // at level l whose particle count exceeds the leaf capacity (ncrit) and whose
 // level is below maxDepth is internal; its children are its non-empty
 // octants.  The node set of the reference's insertion build is exactly this
-// set, independent of insertion order, so it is built here top-down, one
-// level per launch, by splitting each internal node's contiguous key range at
-// its level-l digit boundaries (binary search).  Children of a node are
-// allocated contiguously in ascending octant order.
+// set, independent of insertion order, so it is read off the sorted keys, all
+// levels at once.  Children of a node are contiguous in ascending octant order.
 //
 // Moments (restating Tree.cpp:119-122 running COM, :179-202 maxRadius,
 // :205-254 quadrupoles): leaves sum their members (mass and COM in FP64,
 // quadrupole in FP32 on offsets from the COM); internal nodes combine their
-// children in FP64 (the top-level moment accumulation), bottom-up with
-// per-node arrival counters so each parent is finished by the last child to
-// arrive.
+// children in FP64 (the top-level moment accumulation), level by level.
 #include "engine.cuh"
 #include "walk_common.cuh"
 
@@ -33,227 +29,315 @@ __global__ void reset_counters_kernel(Counters* C) {
     }
 }
 
-__global__ void tree_init_kernel(NodeArrays T, Counters* C, long long n, int leaf_cap, int max_depth) {
-    T.start[0] = 0;
-    T.count[0] = (int)n;
-    T.first_child[0] = -1;
-    T.parent[0] = -1;
-    T.visit[0] = 0;
-    T.nchild[0] = 0;
-    T.level[0] = 0;
-    T.cx[0] = C->root_center[0];
-    T.cy[0] = C->root_center[1];
-    T.cz[0] = C->root_center[2];
-    T.half[0] = C->root_half;
-    T.sysroot[0] = 0;
-    C->next_free = 1;
-    C->level_begin[0] = 0;
-    C->level_begin[1] = 1;
-    C->levels_used = 0;
-    C->max_leaf_count = 0;
+// ---------------------------------------------------------------------------
+// Topology
+// ---------------------------------------------------------------------------
+//
+// Two neighbours in key order say where cells begin, and two particles
+// leaf_cap apart whether a cell is too full, so every particle finds by itself
+// which nodes begin at it, and the tree needs no descent level by level:
+//   a cell of level l begins at particle i if keys i - 1 and i share fewer
+//   than l digits; it holds more than leaf_cap particles if keys i and
+//   i + leaf_cap share at least l;
+//   of the cells that begin at i, c + 1 (one more digit than shared with
+//   i - 1) is a node if its parent, which began earlier, splits; the next is
+//   one if the cell above it splits, and so on: a run [first, top] of levels,
+//   whose last is a leaf.
+// Node numbers are by level and, in a level, in key order, which puts the
+// children of a node side by side in ascending octant order.  A number is a
+// count of runs that reach the level: tree_count counts them per segment of the
+// particles (one warp each), tree_scan adds the segments up, tree_fill hands
+// the numbers out, and tree_finish adds what a node can say for itself.
+//
+// Four launches instead of one per level and six for the leaf list; all of it is
+// latency at small sizes and a read of the keys at large ones.  Before and now
+// (levels and leaf list): 2,048 bodies 92 and 23 us, 1 Mi bodies 217 and 72 us,
+// 4 Mi 293 and 144 us, 16.8 M 537 and 431 us.
+
+constexpr int kRows = kMaxLevels + 1;       // counted per segment: nodes of each level, leaves
+constexpr int kLeafRow = kMaxLevels;
+constexpr int kSegMax = 152 * 48;           // as many warps as stay resident
+constexpr unsigned short kNoRun = 0xFFFFu;  // a particle at which no node begins
+
+static_assert(kRows <= 32, "a lane counts a row");
+
+long long tree_counts_size() { return (long long)kRows * kSegMax + 32; }
+
+// Digits that two keys share, at most `levels`.
+__device__ __forceinline__ int shared_digits(unsigned long long a, unsigned long long b, int levels) {
+    return min((__clzll((long long)(a ^ b)) - 1) / 3, levels);
 }
 
-void launch_tree_init(NodeArrays& T, Counters* C, long long n, int leaf_cap, int max_depth, cudaStream_t s) {
-    tree_init_kernel<<<1, 1, 0, s>>>(T, C, n, leaf_cap, max_depth);
+__device__ __forceinline__ bool share(unsigned long long a, unsigned long long b, int digits) {
+    return ((a ^ b) >> (3 * (kKeyLevels - digits))) == 0;
 }
 
-// First index k in [lo, hi) whose level digit (at `shift`) is >= d.
-__device__ __forceinline__ int digit_lower_bound(const unsigned long long* __restrict__ keys, int lo, int hi,
-                                                 int shift, unsigned d) {
-    while (lo < hi) {
-        const int mid = lo + ((hi - lo) >> 1);
-        const unsigned v = (unsigned)(__ldg(keys + mid) >> shift) & 7u;
-        if (v < d)
-            lo = mid + 1;
-        else
-            hi = mid;
-    }
-    return lo;
-}
-
-constexpr int kLevelThreads = 256;
-
-// One level of the split, eight lanes per node: lane d finds where octant d
-// begins in the node's key range (d = 1..7 by independent binary searches,
-// so the top levels' long ranges cost one search's latency, not seven) and
-// creates child d.  Ensemble (F.sys_levels > 0): levels above sys_levels
-// group systems by id digits, always split and carry no geometry; a child at
-// level sys_levels is a system root and takes that system's cube; below it
-// the reference's recurrence runs from that root.
-__global__ void __launch_bounds__(kLevelThreads) tree_level_kernel(NodeArrays T, Counters* C,
-                                                                   const unsigned long long* __restrict__ keys,
-                                                                   int l, int leaf_cap, int max_depth, Forest F,
-                                                                   int levels) {
-    const int begin = C->level_begin[l];
-    const int end = C->level_begin[l + 1];
-    const int shift = 3 * (kKeyLevels - 1 - l);
-    const bool virt = l < F.sys_levels;                 // this level groups systems
-    const bool sys_child = l + 1 == F.sys_levels;      // children are system roots
-    const int depth_cap = max_depth + F.sys_levels;    // max_depth counts from each system root
+// Ensemble (sys_levels > 0): levels above sys_levels group systems by id
+// digits, always split and carry no geometry; a node of level sys_levels is a
+// system root.  max_depth counts from there (depth_cap from the top).
+__global__ void __launch_bounds__(256, 6) tree_count_kernel(const unsigned long long* __restrict__ keys, long long n,
+                                                           int leaf_cap, int depth_cap, int sys_levels, int levels,
+                                                           int nseg, int seglen, unsigned short* __restrict__ runs,
+                                                           int* __restrict__ counts, Counters* C) {
     const int lane = threadIdx.x & 31;
-    const int d = lane & 7;
-    const unsigned gmask = 0xFFu << (lane & 24);       // the node's eight lanes
-    const long long gid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 3;
-    const long long ngroups = (gridDim.x * (long long)blockDim.x) >> 3;
-    // every lane of a warp runs the same number of iterations (shuffles below)
-    const int span = end - begin;
-    const long long warp0 = gid & ~3ll;
-    for (long long g0 = warp0; g0 < span; g0 += ngroups) {
-        const int node = begin + (int)(g0 + (gid & 3));
-        bool split = false;
-        int s = 0, cnt = 0;
-        if (node < end) {
-            cnt = T.count[node];
-            split = virt || (cnt > leaf_cap && l < depth_cap);  // else it stays a leaf
-            s = T.start[node];
+    const int seg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (seg >= nseg) return;
+    const int deepest = min(depth_cap, levels);
+    const long long lo = (long long)seg * seglen, hi = min(n, lo + seglen);
+    int count = 0;  // of row `lane`
+    for (long long base = lo; base < hi; base += 32) {
+        const long long i = base + lane;
+        const bool valid = i < hi;
+        const unsigned long long key = valid ? keys[i] : 0ull;
+        const unsigned long long prev = valid && i > 0 ? keys[i - 1] : 0ull;
+        const bool has_on = valid && i + leaf_cap < n, has_back = valid && i >= leaf_cap;
+        const unsigned long long on = has_on ? keys[i + leaf_cap] : 0ull;
+        const unsigned long long back = has_back ? keys[i - leaf_cap] : 0ull;
+        const int c = i > 0 ? shared_digits(prev, key, levels) : -1;
+        const int full = has_on ? shared_digits(key, on, levels) : -1;  // cells from i on are too full down to here
+        bool node = valid && c < deepest;
+        if (node && c >= sys_levels && full < c && !(has_back && share(back, key, c))) {
+            // the parent of the first cell: where it begins, and whether that
+            // is leaf_cap before a particle that it still holds
+            long long a = max(0ll, i - leaf_cap + 1), b = i;
+            while (a < b) {
+                const long long mid = (a + b) >> 1;
+                if (share(keys[mid], key, c))
+                    b = mid;
+                else
+                    a = mid + 1;
+            }
+            node = a + leaf_cap < n && share(keys[a + leaf_cap], key, c);
         }
-        const int e = s + cnt;
-        const int bd = split ? (d == 0 ? s : digit_lower_bound(keys, s, e, shift, (unsigned)d)) : 0;
-        int bn = __shfl_down_sync(0xffffffffu, bd, 1, 8);  // where octant d + 1 begins
-        if (d == 7) bn = e;
-        const bool has = split && bn > bd;
-        const unsigned hm = (__ballot_sync(0xffffffffu, has) & gmask) >> (lane & 24);
-        const int nch = __popc(hm);
-        int base = 0;
-        if (split && d == 0) base = atomicAdd(&C->next_free, nch);
-        base = __shfl_sync(0xffffffffu, base, lane & 24, 32);
-        if (!split) continue;
-        if (base + nch > T.cap) {
-            if (d == 0) atomicOr(&C->status, kStNodeOverflow);
-            // The slots of this allocation that still fall inside the pool
-            // become inert records (no particles, no children), so the passes
-            // that scan every node up to the pool's end never read an
-            // unwritten record; the parent stays a leaf.  The walk and the
-            // evaluation do not run on the truncated tree, and the host grows
-            // the pool and builds again.
-            if (has) {
-                const int c = base + __popc(hm & ((1u << d) - 1u));
-                if (c < T.cap) {
-                    T.start[c] = 0;
-                    T.count[c] = 0;
-                    T.first_child[c] = -1;
-                    T.parent[c] = node;
-                    T.visit[c] = 0;
-                    T.nchild[c] = 0;
-                    T.level[c] = (unsigned char)(l + 1);
-                    T.cx[c] = T.cx[node];
-                    T.cy[c] = T.cy[node];
-                    T.cz[c] = T.cz[node];
-                    T.half[c] = 0.0;
-                    T.sysroot[c] = T.sysroot[node];
+        unsigned rows = 0;
+        unsigned short run = kNoRun;
+        if (node) {
+            const int first = c + 1;
+            int top = max(first, min(full + 1, deepest));
+            if (first <= sys_levels) top = max(top, min(sys_levels, deepest));
+            rows = ((2u << top) - (1u << first)) | (1u << kLeafRow);
+            run = (unsigned short)(first << 8 | top);
+            if (full >= top && top < depth_cap) {
+                if (top >= kKeyLevels) {
+                    atomicOr(&C->status, kStDepthLimit);
+                    atomicAdd(&C->depth_limited, 1);
+                } else if (top == levels) {
+                    // the keys were sorted on `levels` digits only: this cell
+                    // would split on an unsorted digit, so the build is redone
+                    // on the full key
+                    atomicOr(&C->status, kStSortDepth);
                 }
             }
-            continue;
         }
-        if (has) {
-            const int c = base + __popc(hm & ((1u << d) - 1u));
-            const int cs = bd, ce = bn;
-            T.start[c] = cs;
-            T.count[c] = ce - cs;
-            T.first_child[c] = -1;
-            T.parent[c] = node;
-            T.visit[c] = 0;
-            T.nchild[c] = 0;
-            T.level[c] = (unsigned char)(l + 1);
-            if (virt) {
-                if (sys_child) {
-                    const int sys = (int)(keys[cs] >> (3 * (kKeyLevels - F.sys_levels)));
-                    T.cx[c] = F.root[4 * sys];
-                    T.cy[c] = F.root[4 * sys + 1];
-                    T.cz[c] = F.root[4 * sys + 2];
-                    T.half[c] = F.root[4 * sys + 3];
-                } else {
-                    T.cx[c] = T.cy[c] = T.cz[c] = 0.0;
-                    T.half[c] = 0.0;
-                }
-                T.sysroot[c] = c;
-            } else {
-                const double pcx = T.cx[node], pcy = T.cy[node], pcz = T.cz[node];
-                const double child_half = 0.5 * T.half[node];
-                T.cx[c] = (d & 1) ? __dadd_rn(pcx, child_half) : __dsub_rn(pcx, child_half);
-                T.cy[c] = (d & 2) ? __dadd_rn(pcy, child_half) : __dsub_rn(pcy, child_half);
-                T.cz[c] = (d & 4) ? __dadd_rn(pcz, child_half) : __dsub_rn(pcz, child_half);
-                T.half[c] = child_half;
-                T.sysroot[c] = T.sysroot[node];
-            }
-            if (l + 1 >= kKeyLevels && ce - cs > leaf_cap && l + 1 < depth_cap) {
-                atomicOr(&C->status, kStDepthLimit);
-                atomicAdd(&C->depth_limited, 1);
-            } else if (l + 1 == levels && ce - cs > leaf_cap && l + 1 < depth_cap) {
-                // the keys were sorted on `levels` digits only: this child
-                // would split on an unsorted digit, so the build is redone on
-                // the full key
-                atomicOr(&C->status, kStSortDepth);
-            }
-        }
-        if (d == 0) {
-            T.first_child[node] = base;
-            T.nchild[node] = (unsigned char)nch;
-            atomicMax(&C->levels_used, l + 1);
+        if (valid) runs[i] = run;
+        for (unsigned any = __reduce_or_sync(0xffffffffu, rows); any; any &= any - 1) {
+            const int l = __ffs((int)any) - 1;
+            const int k = __popc(__ballot_sync(0xffffffffu, (rows >> l) & 1u));
+            if (lane == l) count += k;
         }
     }
-    // The last block to finish publishes where level l+2 begins.
+    if (lane < kRows) counts[lane * nseg + seg] = count;
+}
+
+// Row blockIdx.x of the counts: exclusive scan over the segments, in place, and
+// the row's total.
+__global__ void __launch_bounds__(1024) tree_scan_kernel(int* __restrict__ counts, int nseg, int* __restrict__ totals) {
+    __shared__ int warp_sum[32];
+    int* row = counts + (long long)blockIdx.x * nseg;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    constexpr int kPer = (kSegMax + 1023) / 1024;
+    int v[kPer], sum = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const int at = threadIdx.x * kPer + k;
+        v[k] = at < nseg ? row[at] : 0;
+        sum += v[k];
+    }
+    int all;
+    int before = warp_excl_scan(sum, lane, all);
+    if (lane == 0) warp_sum[w] = all;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const int prev = atomicAdd(&C->done_blocks, 1);
-        if (prev == (int)gridDim.x - 1) {
-            int nf = atomicAdd(&C->next_free, 0);
-            if (nf > T.cap) nf = T.cap;
-            C->level_begin[l + 2] = nf;
-            C->done_blocks = 0;
+    int total;
+    const int base = warp_excl_scan(warp_sum[lane], lane, total);
+    before += __shfl_sync(0xffffffffu, base, w);
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const int at = threadIdx.x * kPer + k;
+        if (at < nseg) row[at] = before;
+        before += v[k];
+    }
+    if (threadIdx.x == 0) totals[blockIdx.x] = total;
+}
+
+// Numbers for the runs: per node its start, level, parent, first child and
+// system root, the leaf list, and for a per-particle walk the leaves that begin
+// before each particle (leaf_before) and at it (leaf_start).
+__global__ void __launch_bounds__(256) tree_fill_kernel(NodeArrays T, Counters* C, long long n, int sys_levels,
+                                                        int nseg, int seglen, const unsigned short* __restrict__ runs,
+                                                        const int* __restrict__ counts,
+                                                        const int* __restrict__ totals, int* __restrict__ leaf_list,
+                                                        unsigned* __restrict__ leaf_before,
+                                                        unsigned* __restrict__ leaf_start) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    const int seg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (seg >= nseg) return;
+    const int in_row = lane < kRows ? totals[lane] : 0;
+    int nodes;
+    const int begin = warp_excl_scan(lane < kMaxLevels ? in_row : 0, lane, nodes);
+    const bool fits = nodes <= T.cap;
+    if (seg == 0) {
+        // A tree too large for the pool is not written: no levels, no leaves;
+        // the walk and the evaluation see the status, and the host grows the
+        // pool and builds again.
+        const unsigned used = __ballot_sync(0xffffffffu, lane < kMaxLevels && in_row > 0);
+        if (lane < kMaxLevels + 2) C->level_begin[lane] = fits ? (lane < kMaxLevels ? begin : nodes) : 0;
+        if (lane == 0) {
+            C->next_free = nodes;
+            C->levels_used = 31 - __clz((int)used);
+            if (!fits) atomicOr(&C->status, kStNodeOverflow);
         }
+        if (lane == kLeafRow) C->nleaves = fits ? in_row : 0;
+    }
+    if (!fits) return;
+    // lane l: the number of the next node of level l (of the next leaf in the list)
+    int next = lane < kRows ? (lane < kMaxLevels ? begin : 0) + counts[lane * nseg + seg] : 0;
+    const long long lo = (long long)seg * seglen, hi = min(n, lo + seglen);
+    for (long long base = lo; base < hi; base += 32) {
+        const long long i = base + lane;
+        const unsigned short run = i < hi ? runs[i] : kNoRun;
+        const bool node = run != kNoRun;
+        const int first = run >> 8, top = run & 0xFF;
+        const unsigned rows = node ? (2u << top) - (1u << first) : 0u;
+        const unsigned leaves = __ballot_sync(0xffffffffu, node);
+        const unsigned at_sys = __ballot_sync(0xffffffffu, node && first <= sys_levels);
+        const int sys_root = __shfl_sync(0xffffffffu, next, sys_levels) + __popc(at_sys & (lt_mask | 1u << lane)) - 1;
+        const int leaf = __shfl_sync(0xffffffffu, next, kLeafRow) + __popc(leaves & lt_mask);
+        if (leaf_before && i < hi) {
+            leaf_before[i] = (unsigned)leaf;
+            leaf_start[i] = node ? 1u : 0u;
+        }
+        int up = -1;         // this particle's node of the level above
+        unsigned at_up = 0;  // the lanes with a node of that level
+        int level_up = -1, begun = lane == kLeafRow ? __popc(leaves) : 0;
+        for (unsigned any = __reduce_or_sync(0xffffffffu, rows); any; any &= any - 1) {
+            const int l = __ffs((int)any) - 1;
+            const unsigned at = __ballot_sync(0xffffffffu, (rows >> l) & 1u);
+            const int next_up = __shfl_sync(0xffffffffu, next, l > 0 ? l - 1 : 0);
+            const int num = __shfl_sync(0xffffffffu, next, l) + __popc(at & lt_mask);
+            if ((rows >> l) & 1u) {
+                // the parent of the first began earlier: the last of its level so far
+                if (l == first) up = l > 0 ? next_up + __popc((level_up == l - 1 ? at_up : 0u) & lt_mask) - 1 : -1;
+                T.start[num] = (int)i;
+                T.level[num] = (unsigned char)l;
+                T.parent[num] = up;
+                if (l > first) T.first_child[up] = num;
+                T.sysroot[num] = l < sys_levels ? num : sys_root;
+                up = num;
+            }
+            if (lane == l) begun = __popc(at);
+            at_up = at;
+            level_up = l;
+        }
+        if (node) {
+            T.first_child[up] = -1;
+            leaf_list[leaf] = up;
+        }
+        next += begun;
     }
 }
 
-void launch_tree_levels(NodeArrays& T, Counters* C, const unsigned long long* keys, long long n, int leaf_cap,
-                        int max_depth, const Forest& F, int levels, cudaStream_t s) {
-    // Enough threads for the widest level (nodes <= cap); levels above it
-    // exit after a bounds check.
-    long long blocks = ((long long)T.cap / 4 * 8 + kLevelThreads - 1) / kLevelThreads;
+// What a node has by itself: its particle count (the end of its key range),
+// child count, centre and size (the reference's recurrence from the root
+// cube, rounded in FP64 as NewChild does).
+__global__ void __launch_bounds__(256) tree_finish_kernel(NodeArrays T, Counters* C,
+                                                         const unsigned long long* __restrict__ keys, long long n,
+                                                         int leaf_cap, Forest F) {
+    const int nodes = C->next_free;
+    if (nodes > T.cap) return;
+    int largest = 0;
+    for (int node = blockIdx.x * blockDim.x + threadIdx.x; node < nodes; node += gridDim.x * blockDim.x) {
+        const int s = T.start[node], l = T.level[node], fc = T.first_child[node];
+        const unsigned long long key = keys[s];
+        long long a = s, b = n;  // a within, b past the end
+        if (l > 0) {
+            for (long long step = leaf_cap; a + step < n; step *= 4) {
+                if (!share(keys[a + step], key, l)) {
+                    b = a + step;
+                    break;
+                }
+                a += step;
+            }
+            while (b - a > 1) {
+                const long long mid = (a + b) >> 1;
+                if (share(keys[mid], key, l))
+                    a = mid;
+                else
+                    b = mid;
+            }
+        }
+        const int count = (int)(b - s);
+        T.count[node] = count;
+        int nch = 0;
+        if (fc >= 0) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) nch += fc + k < nodes && T.parent[fc + k] == node ? 1 : 0;
+        } else {
+            largest = max(largest, count);
+        }
+        T.nchild[node] = (unsigned char)nch;
+        double cx = 0.0, cy = 0.0, cz = 0.0, half = 0.0;
+        if (l >= F.sys_levels) {
+            if (F.sys_levels > 0) {
+                const int sys = (int)(key >> (3 * (kKeyLevels - F.sys_levels)));
+                cx = F.root[4 * sys];
+                cy = F.root[4 * sys + 1];
+                cz = F.root[4 * sys + 2];
+                half = F.root[4 * sys + 3];
+            } else {
+                cx = C->root_center[0];
+                cy = C->root_center[1];
+                cz = C->root_center[2];
+                half = C->root_half;
+            }
+            for (int k = F.sys_levels; k < l; ++k) {
+                const unsigned d = (unsigned)(key >> (3 * (kKeyLevels - 1 - k))) & 7u;
+                half *= 0.5;
+                cx = __dadd_rn(cx, d & 1 ? half : -half);
+                cy = __dadd_rn(cy, d & 2 ? half : -half);
+                cz = __dadd_rn(cz, d & 4 ? half : -half);
+            }
+        }
+        T.cx[node] = cx;
+        T.cy[node] = cy;
+        T.cz[node] = cz;
+        T.half[node] = half;
+    }
+    __shared__ int s_largest;
+    if (threadIdx.x == 0) s_largest = 0;
+    __syncthreads();
+    largest = __reduce_max_sync(0xffffffffu, largest);
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_largest, largest);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_largest > 0) atomicMax(&C->max_leaf_count, s_largest);
+}
+
+int launch_tree(NodeArrays& T, Counters* C, const unsigned long long* keys, long long n, int leaf_cap, int max_depth,
+                const Forest& F, int levels, const TreeBuffers& B, bool leaf_scan, cudaStream_t s) {
+    const int seglen = 32 * (int)((n + 32ll * kSegMax - 1) / (32ll * kSegMax));
+    const int nseg = (int)((n + seglen - 1) / seglen);
+    const unsigned g = (unsigned)((nseg + 7) / 8);
+    int* totals = B.counts + (long long)kRows * kSegMax;
+    const int depth_cap = max_depth < kMaxLevels ? max_depth + F.sys_levels : kMaxLevels + F.sys_levels;
+    tree_count_kernel<<<g, 256, 0, s>>>(keys, n, leaf_cap, depth_cap, F.sys_levels, levels, nseg, seglen, B.runs,
+                                        B.counts, C);
+    tree_scan_kernel<<<kRows, 1024, 0, s>>>(B.counts, nseg, totals);
+    tree_fill_kernel<<<g, 256, 0, s>>>(T, C, n, F.sys_levels, nseg, seglen, B.runs, B.counts, totals, B.leaf_list,
+                                       leaf_scan ? B.leaf_before : nullptr, leaf_scan ? B.leaf_start : nullptr);
+    long long blocks = ((long long)std::min<long long>(T.cap, 2 * n) + 255) / 256;
     if (blocks > 152 * 8) blocks = 152 * 8;
-    if (blocks < 1) blocks = 1;
-    for (int l = 0; l < levels; ++l)
-        tree_level_kernel<<<(unsigned)blocks, kLevelThreads, 0, s>>>(T, C, keys, l, leaf_cap, max_depth, F, levels);
-}
-
-// ---------------------------------------------------------------------------
-// Leaf list in key order
-// ---------------------------------------------------------------------------
-
-__global__ void leaf_mark_kernel(NodeArrays T, Counters* C, long long n, int* __restrict__ leaf_at,
-                                 unsigned* __restrict__ flags) {
-    const int nn = min(C->next_free, T.cap);
-    for (int node = blockIdx.x * blockDim.x + threadIdx.x; node < nn; node += gridDim.x * blockDim.x) {
-        if (T.first_child[node] != -1) continue;
-        const int s = T.start[node];
-        // inert records of an overflowed allocation own no particles
-        if (T.count[node] <= 0 || s < 0 || s >= n) continue;
-        leaf_at[s] = node;
-        flags[s] = 1u;
-        atomicMax(&C->max_leaf_count, T.count[node]);
-    }
-}
-
-__global__ void leaf_compact_kernel(const int* __restrict__ leaf_at, const unsigned* __restrict__ flags,
-                                    const unsigned* __restrict__ pos, long long n, int* __restrict__ leaf_list,
-                                    Counters* C) {
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-        if (flags[k]) leaf_list[pos[k]] = leaf_at[k];
-        if (k == n - 1) C->nleaves = (int)(pos[k] + flags[k]);
-    }
-}
-
-void launch_leaf_list(NodeArrays& T, Counters* C, long long n, int* leaf_at, unsigned* flags, unsigned* scan_out,
-                      int* leaf_list, SortBuffers& sb, cudaStream_t s) {
-    cudaMemsetAsync(flags, 0, sizeof(unsigned) * n, s);
-    long long b1 = ((long long)T.cap + 255) / 256;
-    if (b1 > 152 * 8) b1 = 152 * 8;
-    leaf_mark_kernel<<<(unsigned)b1, 256, 0, s>>>(T, C, n, leaf_at, flags);
-    device_exclusive_scan(flags, scan_out, n, sb.scan_tmp, s);
-    long long b2 = (n + 255) / 256;
-    if (b2 > 152 * 8) b2 = 152 * 8;
-    leaf_compact_kernel<<<(unsigned)b2, 256, 0, s>>>(leaf_at, flags, scan_out, n, leaf_list, C);
+    tree_finish_kernel<<<(unsigned)blocks, 256, 0, s>>>(T, C, keys, n, leaf_cap, F);
+    return 4;
 }
 
 // ---------------------------------------------------------------------------
