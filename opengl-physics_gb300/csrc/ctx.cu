@@ -59,7 +59,7 @@ void free_particles(ngrav_gpu_ctx* ctx) {
     P.cap = 0;
     SortBuffers& S = ctx->SB;
     dfree(S.keys); dfree(S.keys_alt); dfree(S.vals); dfree(S.vals_alt); dfree(S.hist);
-    dfree(S.ktab);
+    dfree(S.frame);
     S.cap = 0;
     TreeBuffers& B = ctx->TB;
     dfree(B.runs); dfree(B.counts); dfree(B.leaf_list); dfree(B.leaf_before); dfree(B.leaf_start);
@@ -92,7 +92,7 @@ int alloc_particles(ngrav_gpu_ctx* ctx, long long n) {
     NG_CUDA(dalloc(S.vals_alt, c));
     S.hist_cap = radix_hist_size(c);
     NG_CUDA(dalloc(S.hist, S.hist_cap));
-    NG_CUDA(dalloc(S.ktab, key_table_entries()));
+    NG_CUDA(dalloc(S.frame, kFrame));
     S.cap = c;
     TreeBuffers& B = ctx->TB;
     NG_CUDA(dalloc(B.runs, c)); NG_CUDA(dalloc(B.counts, tree_counts_size())); NG_CUDA(dalloc(B.leaf_list, c));
@@ -207,14 +207,13 @@ void enqueue_eval(ngrav_gpu_ctx* ctx, bool bbox_ready, bool kick, float hdt) {
         launch_bbox(P.pos, split ? P.plo : nullptr, n, ctx->C, s);
         ctx->launches += 2;
     }
-    launch_root(ctx->C, n, s);
+    launch_root(ctx->C, n, ctx->SB.frame, s);
     if (ctx->F.nsys > 1) {  // ensemble: every system's own root cube
         launch_forest_bbox(P.pos, split ? P.plo : nullptr, n, ctx->F, ctx->C, s);
         launch_forest_root(ctx->F, s);
         ctx->launches += 2;
     }
-    ctx->launches += launch_keys(P.pos, split ? P.plo : nullptr, n, ctx->C, ctx->F, ctx->SB.ktab, ctx->SB.keys,
-                                 ctx->SB.vals, s) - 1;
+    launch_keys(P.pos, split ? P.plo : nullptr, n, ctx->C, ctx->F, ctx->SB.frame, ctx->SB.keys, ctx->SB.vals, s);
     rec(ctx, 1);
     // The keys are sorted on their top `levels` digits only (whole 9-bit
     // passes, so at least that many levels), as deep as the tree went at the

@@ -70,6 +70,7 @@ struct ngrav_gpu_ctx {
     long long* f_off = nullptr;
     double* f_root = nullptr;
     unsigned long long* f_bbox = nullptr;
+    float4* f_frame = nullptr;
     std::vector<long long> h_off;
     // CUDA graphs of one KDK step (kick-drift + force evaluation), keyed by
     // every pointer and parameter the launches bake in; two slots because the

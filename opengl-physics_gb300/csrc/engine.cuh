@@ -182,7 +182,7 @@ struct SortBuffers {
     unsigned* vals_alt = nullptr;
     unsigned* hist = nullptr;         // kRsBins x blocks
     long long hist_cap = 0;
-    long long* ktab = nullptr;        // centres of the top key levels, ordered images (key_table_entries())
+    float4* frame = nullptr;          // key frame of a single system (kFrame)
 };
 
 struct WalkParams {
@@ -214,6 +214,10 @@ struct WalkParams {
     float lm_budget;                  // the budget itself
 };
 
+// A root cube in the form the keys are computed from, kFrame float4 per system:
+// centre high parts, tolerance; centre low parts, scale; scale's low part.
+constexpr int kFrame = 3;
+
 // A forest of independent systems in one particle set (ensemble).  System s
 // holds slots [off[s], off[s+1]) in every tree order; its id occupies the top
 // sys_levels key digits, the remaining 21 - sys_levels digits are the octant
@@ -226,9 +230,28 @@ struct Forest {
     const long long* off = nullptr;   // nsys + 1 slot offsets
     double* root = nullptr;           // per system: centre x, y, z, half (4 doubles)
     unsigned long long* bbox = nullptr;  // per system: encoded min x, y, z, max x, y, z
+    float4* frame = nullptr;          // per system: its key frame (kFrame)
 };
 
-// System of a slot (binary search over the offsets).
+__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
+    s = a + b;
+    const float bb = s - a;
+    e = (a - (s - bb)) + (b - bb);
+}
+
+__device__ __forceinline__ void fast_two_sum(float a, float b, float& s, float& e) {
+    s = a + b;
+    e = b - (s - a);
+}
+
+// Offset of a double-float coordinate (h + l) from a double-float centre
+// (ch + cl), as a normalised double-float pair.
+__device__ __forceinline__ void df_offset(float h, float l, float ch, float cl, float& oh, float& ol) {
+    float s, e;
+    two_sum(h, -ch, s, e);
+    fast_two_sum(s, e + (l - cl), oh, ol);
+}
+
 // (h, l) += d for a double-float pair: error-free two-sum, renormalised.
 __device__ __forceinline__ void df_add(float& h, float& l, float d) {
     const float s = h + d;
@@ -238,6 +261,88 @@ __device__ __forceinline__ void df_add(float& h, float& l, float d) {
     const float h2 = s + l2;
     l = l2 - (h2 - s);
     h = h2;
+}
+
+// Bounding box of double-float coordinates, compared as pairs: the high part is
+// the rounded value, so it orders the values, and the low part does where the
+// high parts are equal.  (FP64 minima and maxima cost a particle a dozen
+// instructions of a pipe 64 times narrower.)
+struct DfBox {
+    float2 lo[3], hi[3];  // (high, low)
+};
+
+__device__ __forceinline__ bool df_less(const float2& a, const float2& b) {
+    return a.x < b.x || (a.x == b.x && a.y < b.y);
+}
+
+__device__ __forceinline__ DfBox empty_box() {
+    DfBox b;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        b.lo[k] = make_float2(1.f / 0.f, 0.f);
+        b.hi[k] = make_float2(-1.f / 0.f, 0.f);
+    }
+    return b;
+}
+
+__device__ __forceinline__ void box_take(DfBox& b, int k, const float2& lo, const float2& hi) {
+    if (df_less(lo, b.lo[k])) b.lo[k] = lo;
+    if (df_less(b.hi[k], hi)) b.hi[k] = hi;
+}
+
+__device__ __forceinline__ void box_add(DfBox& b, const float4& p, const float4& l) {
+    const float2 x = make_float2(p.x, l.x), y = make_float2(p.y, l.y), z = make_float2(p.z, l.z);
+    box_take(b, 0, x, x);
+    box_take(b, 1, y, y);
+    box_take(b, 2, z, z);
+}
+
+__device__ __forceinline__ void box_warp(DfBox& b) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            float2 lo, hi;
+            lo.x = __shfl_xor_sync(0xffffffffu, b.lo[k].x, o);
+            lo.y = __shfl_xor_sync(0xffffffffu, b.lo[k].y, o);
+            hi.x = __shfl_xor_sync(0xffffffffu, b.hi[k].x, o);
+            hi.y = __shfl_xor_sync(0xffffffffu, b.hi[k].y, o);
+            box_take(b, k, lo, hi);
+        }
+    }
+}
+
+// Order-preserving integer image of a double, for atomics.
+__device__ __forceinline__ unsigned long long enc_f64(double d) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(d);
+    return (u & 0x8000000000000000ull) ? ~u : (u | 0x8000000000000000ull);
+}
+
+__device__ __forceinline__ unsigned long long enc_df(const float2& v) { return enc_f64((double)v.x + (double)v.y); }
+
+// The block's box into the counters (all threads call; 256 threads).
+__device__ __forceinline__ void box_publish(DfBox& b, bool bad, Counters* C) {
+    __shared__ float2 s_lo[3][8], s_hi[3][8];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    box_warp(b);
+    if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            s_lo[k][w] = b.lo[k];
+            s_hi[k][w] = b.hi[k];
+        }
+    }
+    bad = __syncthreads_or(bad);
+    if (threadIdx.x < 3) {
+        float2 lo = s_lo[threadIdx.x][0], hi = s_hi[threadIdx.x][0];
+        for (int j = 1; j < 8; ++j) {
+            if (df_less(s_lo[threadIdx.x][j], lo)) lo = s_lo[threadIdx.x][j];
+            if (df_less(hi, s_hi[threadIdx.x][j])) hi = s_hi[threadIdx.x][j];
+        }
+        atomicMin(&C->bbox_min[threadIdx.x], enc_df(lo));
+        atomicMax(&C->bbox_max[threadIdx.x], enc_df(hi));
+    }
+    if (threadIdx.x == 0 && bad) atomicOr(&C->status, kStNonFinite);
 }
 
 // Closing or opening half-kick of one particle: v += h a, as a double-float
@@ -254,6 +359,7 @@ __device__ __forceinline__ void kick_v(float4& v, float4* vl, float h, const flo
     }
 }
 
+// System of a slot (binary search over the offsets).
 __device__ __forceinline__ int forest_system(const Forest& F, long long k) {
     int lo = 0, hi = F.nsys - 1;
     while (lo < hi) {
@@ -268,24 +374,22 @@ __device__ __forceinline__ int forest_system(const Forest& F, long long k) {
 
 // ---- launchers (each enqueues on `s`; no host synchronisation) ----
 void launch_bbox(const float4* pos, const float4* plo, long long n, Counters* C, cudaStream_t s);
-void launch_root(Counters* C, long long n, cudaStream_t s);
+void launch_root(Counters* C, long long n, float4* frame, cudaStream_t s);
 // Ensemble: per-system bounding boxes and root cubes (F.nsys > 1).
 void launch_forest_bbox(const float4* pos, const float4* plo, long long n, const Forest& F, Counters* C,
                         cudaStream_t s);
 void launch_forest_root(const Forest& F, cudaStream_t s);
 void launch_collapse_split(float4* pos, float4* plo, long long n, cudaStream_t s);
-// Keys of the current order (vals = 0 .. n-1); a single system also fills
-// the centre table ktab (key_table_entries() doubles).  Returns the launches made.
-int launch_keys(const float4* pos, const float4* plo, long long n, Counters* C, const Forest& F, long long* ktab,
-                unsigned long long* keys, unsigned* vals, cudaStream_t s);
+// Keys of the current order (vals = 0 .. n-1), in the frames that the root
+// kernels wrote.
+void launch_keys(const float4* pos, const float4* plo, long long n, Counters* C, const Forest& F, const float4* frame,
+                 unsigned long long* keys, unsigned* vals, cudaStream_t s);
 // Stable LSD radix sort of (keys, vals) over bits [shift0, shift0 + kRsDigitBits*passes);
 // result ends in (keys, vals) (the alternates are scratch).
 void radix_sort_pairs(SortBuffers& sb, long long n, int passes, int shift0, cudaStream_t s);
 // Entries of SortBuffers::hist for n keys: the tile histograms, then the
 // digit totals.
 long long radix_hist_size(long long n);
-// Doubles of SortBuffers::ktab: the tabulated key centres of the three axes.
-long long key_table_entries();
 void launch_permute(const Particles& P, const unsigned* perm, long long n, bool split, cudaStream_t s);
 // Builds the nodes down to level `levels` (keys sorted on their top `levels`
 // digits; a node there that would still split sets kStSortDepth) and the leaf

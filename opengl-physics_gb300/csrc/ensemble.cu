@@ -210,6 +210,7 @@ void free_forest(ngrav_gpu_ctx* ctx) {
     dfree(ctx->f_off);
     dfree(ctx->f_root);
     dfree(ctx->f_bbox);
+    dfree(ctx->f_frame);
     ctx->F = Forest{};
     ctx->h_off.clear();
 }
@@ -236,6 +237,7 @@ int ngrav_gpu_set_ensemble(ngrav_gpu_ctx* ctx, int nsys, const int64_t* offsets)
     NG_CUDA(dalloc(ctx->f_off, nsys + 1));
     NG_CUDA(dalloc(ctx->f_root, 4LL * nsys));
     NG_CUDA(dalloc(ctx->f_bbox, 6LL * nsys));
+    NG_CUDA(dalloc(ctx->f_frame, (long long)kFrame * nsys));
     std::vector<long long> off(offsets, offsets + nsys + 1);
     std::vector<unsigned long long> box(6LL * nsys);
     for (int s = 0; s < nsys; ++s)
@@ -251,6 +253,7 @@ int ngrav_gpu_set_ensemble(ngrav_gpu_ctx* ctx, int nsys, const int64_t* offsets)
     ctx->F.off = ctx->f_off;
     ctx->F.root = ctx->f_root;
     ctx->F.bbox = ctx->f_bbox;
+    ctx->F.frame = ctx->f_frame;
     ctx->primed = false;
     ctx->acc_valid = false;
     return NGRAV_OK;

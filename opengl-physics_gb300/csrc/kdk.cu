@@ -20,11 +20,6 @@
 
 namespace ngrav {
 
-__device__ __forceinline__ unsigned long long enc_f64_k(double d) {
-    const unsigned long long u = (unsigned long long)__double_as_longlong(d);
-    return (u & 0x8000000000000000ull) ? ~u : (u | 0x8000000000000000ull);
-}
-
 // ---------------------------------------------------------------------------
 // Upload / download
 // ---------------------------------------------------------------------------
@@ -207,8 +202,7 @@ __global__ void __launch_bounds__(256) kick_drift_kernel(long long n, float4* __
                                                          float4* __restrict__ plo, float4* __restrict__ vel,
                                                          float4* __restrict__ vlo, const float4* __restrict__ acc,
                                                          float hdt, float dt, Counters* C) {
-    double lo[3] = {1.0 / 0.0, 1.0 / 0.0, 1.0 / 0.0};
-    double hi[3] = {-1.0 / 0.0, -1.0 / 0.0, -1.0 / 0.0};
+    DfBox box = empty_box();
     bool bad = false;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         float4 v = vel[i];
@@ -218,9 +212,9 @@ __global__ void __launch_bounds__(256) kick_drift_kernel(long long n, float4* __
         vel[i] = v;
         if (SPLIT) vlo[i] = vl;
         float4 p = pos[i];
-        double q[3];
+        float4 l = make_float4(0.f, 0.f, 0.f, 0.f);
         if (SPLIT) {
-            float4 l = plo[i];
+            l = plo[i];
             float* ph = &p.x;
             float* pl = &l.x;
             const float dv[3] = {fmaf(dt, v.x, dt * vl.x), fmaf(dt, v.y, dt * vl.y), fmaf(dt, v.z, dt * vl.z)};
@@ -234,51 +228,18 @@ __global__ void __launch_bounds__(256) kick_drift_kernel(long long n, float4* __
                 const float h2 = s + lo2;
                 pl[k] = lo2 - (h2 - s);
                 ph[k] = h2;
-                q[k] = (double)ph[k] + (double)pl[k];
             }
             plo[i] = l;
         } else {
             p.x = fmaf(dt, v.x, p.x);
             p.y = fmaf(dt, v.y, p.y);
             p.z = fmaf(dt, v.z, p.z);
-            q[0] = p.x;
-            q[1] = p.y;
-            q[2] = p.z;
         }
         pos[i] = p;
         bad |= !(isfinite(p.x) && isfinite(p.y) && isfinite(p.z));
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            lo[k] = fmin(lo[k], q[k]);
-            hi[k] = fmax(hi[k], q[k]);
-        }
+        box_add(box, p, l);
     }
-    __shared__ double slo[3][8], shi[3][8];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        double l = lo[k], h = hi[k];
-        for (int o = 16; o > 0; o >>= 1) {
-            l = fmin(l, __shfl_xor_sync(0xffffffffu, l, o));
-            h = fmax(h, __shfl_xor_sync(0xffffffffu, h, o));
-        }
-        if (lane == 0) {
-            slo[k][w] = l;
-            shi[k][w] = h;
-        }
-    }
-    bad = __syncthreads_or(bad);
-    if (threadIdx.x < 3) {
-        const int k = threadIdx.x;
-        double l = slo[k][0], h = shi[k][0];
-        for (int j = 1; j < 8; ++j) {
-            l = fmin(l, slo[k][j]);
-            h = fmax(h, shi[k][j]);
-        }
-        atomicMin(&C->bbox_min[k], enc_f64_k(l));
-        atomicMax(&C->bbox_max[k], enc_f64_k(h));
-    }
-    if (threadIdx.x == 0 && bad) atomicOr(&C->status, kStNonFinite);
+    box_publish(box, bad, C);
 }
 
 void launch_kick_drift(const Particles& P, long long n, float hdt, float dt, bool split, Counters* C,

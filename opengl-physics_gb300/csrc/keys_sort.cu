@@ -22,22 +22,9 @@ namespace ngrav {
 // FP64 bounding box with order-preserving integer atomics
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ unsigned long long enc_f64(double d) {
-    const unsigned long long u = (unsigned long long)__double_as_longlong(d);
-    return (u & 0x8000000000000000ull) ? ~u : (u | 0x8000000000000000ull);
-}
-
 __device__ __forceinline__ double dec_f64(unsigned long long u) {
     u = (u & 0x8000000000000000ull) ? (u & 0x7FFFFFFFFFFFFFFFull) : ~u;
     return __longlong_as_double((long long)u);
-}
-
-__device__ __forceinline__ double pos_d(const float4& hi, const float4* plo, long long i, int axis) {
-    const float h = axis == 0 ? hi.x : (axis == 1 ? hi.y : hi.z);
-    if (!plo) return (double)h;
-    const float4 lo = plo[i];
-    const float l = axis == 0 ? lo.x : (axis == 1 ? lo.y : lo.z);
-    return (double)h + (double)l;
 }
 
 constexpr int kBoxThreads = 256;
@@ -45,47 +32,36 @@ constexpr int kBoxThreads = 256;
 __global__ void __launch_bounds__(kBoxThreads) bbox_kernel(const float4* __restrict__ pos,
                                                            const float4* __restrict__ plo, long long n,
                                                            Counters* C) {
-    double lo[3] = {1.0 / 0.0, 1.0 / 0.0, 1.0 / 0.0};
-    double hi[3] = {-1.0 / 0.0, -1.0 / 0.0, -1.0 / 0.0};
+    DfBox box = empty_box();
     bool bad = false;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const float4 p = pos[i];
         bad |= !(isfinite(p.x) && isfinite(p.y) && isfinite(p.z) && isfinite(p.w));
-        for (int a = 0; a < 3; ++a) {
-            const double v = pos_d(p, plo, i, a);
-            lo[a] = fmin(lo[a], v);
-            hi[a] = fmax(hi[a], v);
-        }
+        box_add(box, p, plo ? plo[i] : make_float4(0.f, 0.f, 0.f, 0.f));
     }
-    __shared__ double slo[3][kBoxThreads / 32], shi[3][kBoxThreads / 32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int a = 0; a < 3; ++a) {
-        double l = lo[a], h = hi[a];
-        for (int o = 16; o > 0; o >>= 1) {
-            l = fmin(l, __shfl_xor_sync(0xffffffffu, l, o));
-            h = fmax(h, __shfl_xor_sync(0xffffffffu, h, o));
-        }
-        if (lane == 0) {
-            slo[a][w] = l;
-            shi[a][w] = h;
-        }
-    }
-    bad = __syncthreads_or(bad);
-    if (threadIdx.x < 3) {
-        const int a = threadIdx.x;
-        double l = slo[a][0], h = shi[a][0];
-        for (int k = 1; k < kBoxThreads / 32; ++k) {
-            l = fmin(l, slo[a][k]);
-            h = fmax(h, shi[a][k]);
-        }
-        atomicMin(&C->bbox_min[a], enc_f64(l));
-        atomicMax(&C->bbox_max[a], enc_f64(h));
-    }
-    if (threadIdx.x == 0 && bad) atomicOr(&C->status, kStNonFinite);
+    box_publish(box, bad, C);
+}
+
+// The key frame of a root cube: its centre as double-float, the scale
+// 2^(digits - 1) / half to cells of the finest level, and how near a cell's face
+// (in cells) the arithmetic of axis_cell leaves the side in doubt.  The offset
+// from the centre is good to 2^-47 (|centre| + half), its product with the scale
+// to 2^-46, and the reference's centres are within 21 roundings of the grid: all
+// below 2^-23 (1 + |centre| / half) cells.  A scale whose low part would
+// underflow is not used.
+__device__ void write_frame(float4* f, double cx, double cy, double cz, double half, int digits) {
+    const float hx = (float)cx, hy = (float)cy, hz = (float)cz;
+    const double scale = (double)(1 << (digits - 1)) / half;
+    const float sh = (float)scale;
+    const double far = fmax(fmax(fabs(cx), fabs(cy)), fabs(cz)) / half;
+    const float tol = sh > 1e-25f ? (float)(0x1p-20 * (1.0 + far)) : 2.f;
+    f[0] = make_float4(hx, hy, hz, tol);
+    f[1] = make_float4((float)(cx - (double)hx), (float)(cy - (double)hy), (float)(cz - (double)hz), sh);
+    f[2] = make_float4((float)(scale - (double)sh), 0.f, 0.f, 0.f);
 }
 
 // Root cube of BuildRoot (Tree.cpp:54-88), once per evaluation.
-__global__ void root_kernel(Counters* C, long long n) {
+__global__ void root_kernel(Counters* C, long long n, float4* frame) {
     double lo[3], hi[3];
     for (int a = 0; a < 3; ++a) {
         lo[a] = n > 0 ? dec_f64(C->bbox_min[a]) : 0.0;
@@ -99,6 +75,7 @@ __global__ void root_kernel(Counters* C, long long n) {
     if (!(half > 1e-12)) half = 1.0;
     for (int a = 0; a < 3; ++a) C->root_center[a] = __dmul_rn(0.5, __dadd_rn(lo[a], hi[a]));
     C->root_half = __dmul_rn(half, 1.001);
+    write_frame(frame, C->root_center[0], C->root_center[1], C->root_center[2], C->root_half, kKeyLevels);
 }
 
 void launch_bbox(const float4* pos, const float4* plo, long long n, Counters* C, cudaStream_t s) {
@@ -108,7 +85,9 @@ void launch_bbox(const float4* pos, const float4* plo, long long n, Counters* C,
     bbox_kernel<<<(unsigned)blocks, kBoxThreads, 0, s>>>(pos, plo, n, C);
 }
 
-void launch_root(Counters* C, long long n, cudaStream_t s) { root_kernel<<<1, 1, 0, s>>>(C, n); }
+void launch_root(Counters* C, long long n, float4* frame, cudaStream_t s) {
+    root_kernel<<<1, 1, 0, s>>>(C, n, frame);
+}
 
 // Ensemble: per-system FP64 bounding boxes.  Slots are grouped by system, so a
 // warp whose 32 slots share one system reduces in registers first; mixed warps
@@ -123,28 +102,22 @@ __global__ void __launch_bounds__(kBoxThreads) forest_bbox_kernel(const float4* 
         const long long i = base + lane;
         const bool has = i < n;
         int sys = has ? forest_system(F, i) : -1;
-        double v[3] = {0.0, 0.0, 0.0};
+        DfBox box = empty_box();
         if (has) {
             const float4 p = pos[i];
             bad |= !(isfinite(p.x) && isfinite(p.y) && isfinite(p.z) && isfinite(p.w));
-            for (int a = 0; a < 3; ++a) v[a] = pos_d(p, plo, i, a);
+            box_add(box, p, plo ? plo[i] : make_float4(0.f, 0.f, 0.f, 0.f));
         }
         const int s0 = __shfl_sync(0xffffffffu, sys, 0);
         const bool uniform = __all_sync(0xffffffffu, !has || sys == s0);
-        for (int a = 0; a < 3; ++a) {
-            double l = has ? v[a] : 1.0 / 0.0, h = has ? v[a] : -1.0 / 0.0;
-            if (uniform) {
-                for (int o = 16; o > 0; o >>= 1) {
-                    l = fmin(l, __shfl_xor_sync(0xffffffffu, l, o));
-                    h = fmax(h, __shfl_xor_sync(0xffffffffu, h, o));
-                }
-                if (lane == 0) {
-                    atomicMin(&F.bbox[6 * s0 + a], enc_f64(l));
-                    atomicMax(&F.bbox[6 * s0 + 3 + a], enc_f64(h));
-                }
-            } else if (has) {
-                atomicMin(&F.bbox[6 * sys + a], enc_f64(l));
-                atomicMax(&F.bbox[6 * sys + 3 + a], enc_f64(h));
+        if (uniform) {
+            box_warp(box);
+            sys = s0;
+        }
+        if (uniform ? lane == 0 : has) {
+            for (int a = 0; a < 3; ++a) {
+                atomicMin(&F.bbox[6 * sys + a], enc_df(box.lo[a]));
+                atomicMax(&F.bbox[6 * sys + 3 + a], enc_df(box.hi[a]));
             }
         }
     }
@@ -171,6 +144,8 @@ __global__ void forest_root_kernel(Forest F) {
         if (!(half > 1e-12)) half = 1.0;
         for (int a = 0; a < 3; ++a) F.root[4 * sys + a] = __dmul_rn(0.5, __dadd_rn(lo[a], hi[a]));
         F.root[4 * sys + 3] = __dmul_rn(half, 1.001);
+        write_frame(F.frame + kFrame * sys, F.root[4 * sys], F.root[4 * sys + 1], F.root[4 * sys + 2],
+                    F.root[4 * sys + 3], kKeyLevels - F.sys_levels);
     }
 }
 
@@ -239,89 +214,30 @@ __device__ __forceinline__ unsigned axis_bits(double p, double c, double h) {
     return bits;
 }
 
-constexpr int kKeyTabLevels = 17;                // key levels whose centres are tabulated per build
-constexpr int kKeyTabSize = 1 << kKeyTabLevels;  // table entries per axis (entry 0 unused)
-constexpr int kKeySub = 4;                       // levels a table thread fills below its own entry
-constexpr int kKeyTop = kKeyTabLevels - 1 - kKeySub;  // level of those threads' entries
-static_assert(kKeyTop >= 0, "the table is deeper than one thread's subtree");
-
-long long key_table_entries() { return 3LL * kKeyTabSize; }
-
-__device__ __forceinline__ double centre_step(double c, long long hb, bool up) {
-    return __dadd_rn(c, __longlong_as_double(up ? hb : (hb | (long long)0x8000000000000000ull)));
-}
-
-// The centre recurrence of an axis depends only on that axis's own octant
-// bits, so the centres of levels 0 .. kKeyTabLevels-1 are tabulated once per
-// build: an implicit binary tree per axis, entry 1 the root centre and entry
-// 2e + b the child of entry e on side b (b = 1: p >= c).  Every entry is the
-// exact FP64 sequence of additions of the walk down to it, so the keys kernel
-// looks the top levels up and adds in FP64 only below them.  One thread per
-// entry of level kKeyTop replays the walk to it and derives its subtree
-// kKeySub levels down, one addition per entry from the parent's value (the
-// same operands and rounding as the walk); one thread per entry above
-// kKeyTop replays its own walk.  Entries are stored as their ordered bit
-// images (ordered_bits), the form the keys kernel compares.
-__global__ void __launch_bounds__(256) key_table_kernel(const Counters* __restrict__ C, long long* __restrict__ tab) {
-    constexpr int nroot = 1 << kKeyTop;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool sub = i < 3 * nroot;
-    const int j = sub ? i : i - 3 * nroot;
-    if (j >= 3 * nroot) return;
-    const int axis = j / nroot;
-    const int e = sub ? nroot + j % nroot : j % nroot;  // an entry of level kKeyTop, or one above it
-    if (e == 0) return;
-    const int l = 31 - __clz(e);  // level of entry e: its bits below the leading one are levels 0 .. l-1
-    double c = C->root_center[axis];
-    long long hb = __double_as_longlong(C->root_half);
-    for (int k = l - 1; k >= 0; --k) {
-        hb -= 1ll << 52;
-        c = centre_step(c, hb, (e >> k) & 1);
+// Cell of the finest of `digits` levels along one axis, without the FP64 pipe:
+// the double-float offset from the root's centre times the scale, split into
+// its whole part and fraction.  A cell's bits are the reference's octant bits
+// unless a face is within the frame's tolerance, which `doubt` reports; then the
+// centre recurrence decides (axis_bits).  In doubt is about one particle in
+// 170,000 of a system around its origin.
+__device__ __forceinline__ unsigned axis_cell(float h, float l, float ch, float cl, float sh, float sl, float tol,
+                                              int digits, bool& doubt) {
+    float oh, ol;
+    df_offset(h, l, ch, cl, oh, ol);
+    const float p = __fmul_rn(oh, sh);
+    const float e = fmaf(oh, sh, -p) + fmaf(oh, sl, ol * sh);
+    const float whole = floorf(p);
+    float f = (p - whole) + e;
+    int q = (int)whole + (1 << (digits - 1));
+    if (f < 0.f) {
+        f += 1.f;
+        q -= 1;
+    } else if (f >= 1.f) {
+        f -= 1.f;
+        q += 1;
     }
-    long long* t = tab + (long long)axis * kKeyTabSize;
-    t[e] = ordered_bits(c);
-    if (!sub) return;
-    double lv[1 << kKeySub];  // the subtree's centres of one level, left to right
-    lv[0] = c;
-#pragma unroll
-    for (int d = 1; d <= kKeySub; ++d) {
-        hb -= 1ll << 52;
-#pragma unroll
-        for (int q = (1 << d) - 1; q >= 0; --q) lv[q] = centre_step(lv[q >> 1], hb, q & 1);
-#pragma unroll
-        for (int q = 0; q < (1 << d); ++q) t[(e << d) + q] = ordered_bits(lv[q]);
-    }
-}
-
-// The double of an ordered bit image (a -0 centre comes back as +0, which
-// gives the same sums with the nonzero halves added to it).
-__device__ __forceinline__ double from_ordered(long long o) {
-    return __longlong_as_double(o ^ ((o >> 63) & 0x7FFFFFFFFFFFFFFFll));
-}
-
-// axis_bits over all kKeyLevels levels with the top kKeyTabLevels looked up
-// in the axis's table of ordered images.
-__device__ __forceinline__ unsigned axis_bits_tab(double p, const long long* __restrict__ tab, double h0) {
-    const long long op = ordered_bits(p);
-    unsigned e = 1;
-#pragma unroll
-    for (int l = 0; l < kKeyTabLevels; ++l) e = 2 * e + (op >= __ldg(tab + e) ? 1u : 0u);
-    // continue from the centre of level kKeyTabLevels: the last tabulated
-    // centre plus or minus h / 2^kKeyTabLevels, as the recurrence would
-    long long hb = __double_as_longlong(h0) - ((long long)kKeyTabLevels << 52);
-    double c = __dadd_rn(from_ordered(__ldg(tab + (e >> 1))),
-                         __longlong_as_double(e & 1 ? hb : (hb | (long long)0x8000000000000000ull)));
-    unsigned bits = e - (1u << kKeyTabLevels);
-#pragma unroll
-    for (int l = kKeyTabLevels; l < kKeyLevels; ++l) {
-        const bool b = op >= ordered_bits(c);
-        bits = (bits << 1) | (b ? 1u : 0u);
-        if (l + 1 < kKeyLevels) {
-            hb -= 1ll << 52;
-            c = __dadd_rn(c, __longlong_as_double(b ? hb : (hb | (long long)0x8000000000000000ull)));
-        }
-    }
-    return bits;
+    doubt |= !(f > tol && f < 1.f - tol) || (unsigned)q >= (1u << digits);
+    return (unsigned)q;
 }
 
 // Spread 21 bits so bit k lands at 3k.
@@ -335,76 +251,58 @@ __device__ __forceinline__ unsigned long long spread3(unsigned v) {
     return x;
 }
 
+// Keys: the system id in the top SYSL digits (none for a single system), then
+// 21 - SYSL levels of octant path from the system's root cube.  Reads of the
+// positions and writes of the keys bound it; the centre recurrence in FP64 for
+// every particle, with the top 17 levels tabulated per build, was bound by the
+// FP64 pipe.  Box, root and keys together, before and now: 2,048 bodies 41 and
+// 20 us, 4 Mi bodies 347 and 103 us, 16.8 M 1,264 and 332 us, 64 systems of
+// 955 k bodies 276 and 119 us.
+template <int SYSL>
 __global__ void __launch_bounds__(256) keys_kernel(const float4* __restrict__ pos, const float4* __restrict__ plo,
-                                                   long long n, const Counters* __restrict__ C,
-                                                   const long long* __restrict__ tab,
+                                                   long long n, const Counters* __restrict__ C, Forest F,
+                                                   const float4* __restrict__ frame,
                                                    unsigned long long* __restrict__ keys,
                                                    unsigned* __restrict__ vals) {
-    const double h0 = C->root_half;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float4 p = pos[i];
-        double px = p.x, py = p.y, pz = p.z;
-        if (plo) {
-            const float4 l = plo[i];
-            px += (double)l.x;
-            py += (double)l.y;
-            pz += (double)l.z;
-        }
-        const unsigned bx = axis_bits_tab(px, tab, h0);
-        const unsigned by = axis_bits_tab(py, tab + kKeyTabSize, h0);
-        const unsigned bz = axis_bits_tab(pz, tab + 2 * kKeyTabSize, h0);
-        keys[i] = spread3(bx) | (spread3(by) << 1) | (spread3(bz) << 2);
-        vals[i] = (unsigned)i;
-    }
-}
-
-// Ensemble keys: the system id in the top SYSL digits, then 21 - SYSL levels
-// of octant path from the system's own root cube.
-template <int SYSL>
-__global__ void __launch_bounds__(256) forest_keys_kernel(const float4* __restrict__ pos,
-                                                          const float4* __restrict__ plo, long long n, Forest F,
-                                                          unsigned long long* __restrict__ keys,
-                                                          unsigned* __restrict__ vals) {
     constexpr int L = kKeyLevels - SYSL;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int sys = forest_system(F, i);
-        const double cx = F.root[4 * sys], cy = F.root[4 * sys + 1], cz = F.root[4 * sys + 2];
-        const double h0 = F.root[4 * sys + 3];
+        const int sys = SYSL > 0 ? forest_system(F, i) : 0;
         const float4 p = pos[i];
-        double px = p.x, py = p.y, pz = p.z;
-        if (plo) {
-            const float4 l = plo[i];
-            px += (double)l.x;
-            py += (double)l.y;
-            pz += (double)l.z;
+        const float4 l = plo ? plo[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 f0 = frame[kFrame * sys], f1 = frame[kFrame * sys + 1];
+        const float sl = frame[kFrame * sys + 2].x;
+        bool doubt = false;
+        unsigned bx = axis_cell(p.x, l.x, f0.x, f1.x, f1.w, sl, f0.w, L, doubt);
+        unsigned by = axis_cell(p.y, l.y, f0.y, f1.y, f1.w, sl, f0.w, L, doubt);
+        unsigned bz = axis_cell(p.z, l.z, f0.z, f1.z, f1.w, sl, f0.w, L, doubt);
+        if (doubt) {
+            const double* root = SYSL > 0 ? F.root + 4 * sys : C->root_center;
+            const double h0 = SYSL > 0 ? root[3] : C->root_half;
+            bx = axis_bits<L>((double)p.x + (double)l.x, root[0], h0);
+            by = axis_bits<L>((double)p.y + (double)l.y, root[1], h0);
+            bz = axis_bits<L>((double)p.z + (double)l.z, root[2], h0);
         }
-        const unsigned bx = axis_bits<L>(px, cx, h0);
-        const unsigned by = axis_bits<L>(py, cy, h0);
-        const unsigned bz = axis_bits<L>(pz, cz, h0);
-        keys[i] = ((unsigned long long)sys << (3 * L)) | spread3(bx) | (spread3(by) << 1) | (spread3(bz) << 2);
+        const unsigned long long id = SYSL > 0 ? (unsigned long long)sys << (3 * L % 64) : 0ull;
+        keys[i] = id | spread3(bx) | (spread3(by) << 1) | (spread3(bz) << 2);
         vals[i] = (unsigned)i;
     }
 }
 
-int launch_keys(const float4* pos, const float4* plo, long long n, Counters* C, const Forest& F, long long* ktab,
-                unsigned long long* keys, unsigned* vals, cudaStream_t s) {
+void launch_keys(const float4* pos, const float4* plo, long long n, Counters* C, const Forest& F, const float4* frame,
+                 unsigned long long* keys, unsigned* vals, cudaStream_t s) {
     long long blocks = (n + 255) / 256;
     if (blocks > 152 * 16) blocks = 152 * 16;
     if (blocks < 1) blocks = 1;
     const unsigned g = (unsigned)blocks;
     switch (F.sys_levels) {
-        case 0:
-            key_table_kernel<<<(6 * (1 << kKeyTop) + 255) / 256, 256, 0, s>>>(C, ktab);
-            keys_kernel<<<g, 256, 0, s>>>(pos, plo, n, C, ktab, keys, vals);
-            return 2;
-        case 1: forest_keys_kernel<1><<<g, 256, 0, s>>>(pos, plo, n, F, keys, vals); break;
-        case 2: forest_keys_kernel<2><<<g, 256, 0, s>>>(pos, plo, n, F, keys, vals); break;
-        case 3: forest_keys_kernel<3><<<g, 256, 0, s>>>(pos, plo, n, F, keys, vals); break;
-        case 4: forest_keys_kernel<4><<<g, 256, 0, s>>>(pos, plo, n, F, keys, vals); break;
-        case 5: forest_keys_kernel<5><<<g, 256, 0, s>>>(pos, plo, n, F, keys, vals); break;
-        default: forest_keys_kernel<6><<<g, 256, 0, s>>>(pos, plo, n, F, keys, vals); break;
+        case 0: keys_kernel<0><<<g, 256, 0, s>>>(pos, plo, n, C, F, frame, keys, vals); break;
+        case 1: keys_kernel<1><<<g, 256, 0, s>>>(pos, plo, n, C, F, F.frame, keys, vals); break;
+        case 2: keys_kernel<2><<<g, 256, 0, s>>>(pos, plo, n, C, F, F.frame, keys, vals); break;
+        case 3: keys_kernel<3><<<g, 256, 0, s>>>(pos, plo, n, C, F, F.frame, keys, vals); break;
+        case 4: keys_kernel<4><<<g, 256, 0, s>>>(pos, plo, n, C, F, F.frame, keys, vals); break;
+        case 5: keys_kernel<5><<<g, 256, 0, s>>>(pos, plo, n, C, F, F.frame, keys, vals); break;
+        default: keys_kernel<6><<<g, 256, 0, s>>>(pos, plo, n, C, F, F.frame, keys, vals); break;
     }
-    return 1;
 }
 
 // Block-wide exclusive scan of one value per thread; returns the block total.

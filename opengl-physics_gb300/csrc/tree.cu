@@ -384,25 +384,6 @@ __device__ __forceinline__ void write_walk_record(NodeArrays& T, int node, doubl
 // of a leaf counts, one where there are many, which spares the reductions.
 // Before and now: 297 k leaves (4 Mi bodies) 278 and 156 us, 462 leaves (2,048
 // bodies) 27 and 13 us; eight lanes throughout took 185 us at 297 k leaves.
-__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
-    s = a + b;
-    const float bb = s - a;
-    e = (a - (s - bb)) + (b - bb);
-}
-
-__device__ __forceinline__ void fast_two_sum(float a, float b, float& s, float& e) {
-    s = a + b;
-    e = b - (s - a);
-}
-
-// Offset of a double-float coordinate (h + l) from a double-float centre
-// (ch + cl), as a normalised double-float pair.
-__device__ __forceinline__ void df_offset(float h, float l, float ch, float cl, float& oh, float& ol) {
-    float s, e;
-    two_sum(h, -ch, s, e);
-    fast_two_sum(s, e + (l - cl), oh, ol);
-}
-
 // (Sh, Sl) += m * (oh + ol), the product of the high parts exact.
 __device__ __forceinline__ void df_add_prod(float& Sh, float& Sl, float m, float oh, float ol) {
     const float p = m * oh;
