@@ -213,21 +213,22 @@ void enqueue_eval(ngrav_gpu_ctx* ctx, bool bbox_ready, bool kick, float hdt) {
         launch_forest_root(ctx->F, s);
         ctx->launches += 2;
     }
-    launch_keys(P.pos, split ? P.plo : nullptr, n, ctx->C, ctx->F, ctx->SB.frame, ctx->SB.keys, ctx->SB.vals, s);
-    rec(ctx, 1);
     // The keys are sorted on their top `levels` digits only (whole 9-bit
     // passes, so at least that many levels), as deep as the tree went at the
     // last evaluation plus a level; a node at the deepest sorted level that
     // would still split stops the build (kStSortDepth) and the evaluation
-    // is redone on the full key.
+    // is redone on the full key.  An ensemble sorts the full key: its systems come
+    // out in the order that each would have alone, whatever the others' depth.
     const int levels = ctx->F.nsys > 1 ? kKeyLevels : ctx->sort_levels;
     const int passes = std::min(kRsPasses, (3 * levels + kRsDigitBits - 1) / kRsDigitBits);
-    radix_sort_pairs(ctx->SB, n, passes, 3 * kKeyLevels - kRsDigitBits * passes, s);
+    const bool alt = sort_from_alt(n, passes);
+    launch_keys(P.pos, split ? P.plo : nullptr, n, ctx->C, ctx->F, ctx->SB.frame,
+                alt ? ctx->SB.keys_alt : ctx->SB.keys, alt ? ctx->SB.vals_alt : ctx->SB.vals, s);
+    rec(ctx, 1);
+    ctx->launches += radix_sort_pairs(ctx->SB, n, passes, 3 * kKeyLevels - kRsDigitBits * passes, s);
     ctx->sort_passes = passes;
     launch_permute(P, ctx->SB.vals, n, split, s);
-    // root, keys, 3 per sort pass (histogram, digit scans, scatter), permute,
-    // walk
-    ctx->launches += 2 + (n > 1 ? 3 * passes : 0) + 1 + 1;
+    ctx->launches += 4;  // root, keys, permute, walk
     std::swap(P.pos, P.pos2);
     std::swap(P.plo, P.plo2);
     std::swap(P.vel, P.vel2);

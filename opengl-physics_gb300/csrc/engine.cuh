@@ -384,9 +384,11 @@ void launch_collapse_split(float4* pos, float4* plo, long long n, cudaStream_t s
 // kernels wrote.
 void launch_keys(const float4* pos, const float4* plo, long long n, Counters* C, const Forest& F, const float4* frame,
                  unsigned long long* keys, unsigned* vals, cudaStream_t s);
-// Stable LSD radix sort of (keys, vals) over bits [shift0, shift0 + kRsDigitBits*passes);
-// result ends in (keys, vals) (the alternates are scratch).
-void radix_sort_pairs(SortBuffers& sb, long long n, int passes, int shift0, cudaStream_t s);
+// Stable LSD radix sort over bits [shift0, shift0 + kRsDigitBits*passes) of the
+// pairs in (keys, vals), or in (keys_alt, vals_alt) where sort_from_alt says so;
+// the result ends in (keys, vals).  Returns the number of launches.
+bool sort_from_alt(long long n, int passes);
+int radix_sort_pairs(SortBuffers& sb, long long n, int passes, int shift0, cudaStream_t s);
 // Entries of SortBuffers::hist for n keys: the tile histograms, then the
 // digit totals.
 long long radix_hist_size(long long n);
