@@ -54,7 +54,6 @@ struct Counters {
     unsigned status;
     int next_free;                    // node allocator
     int level_begin[kMaxLevels + 2];
-    int done_blocks;
     int nleaves;
     int max_leaf_count;
     int depth_limited;
