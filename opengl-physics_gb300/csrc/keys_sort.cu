@@ -332,7 +332,7 @@ __device__ __forceinline__ unsigned block_exclusive_scan(unsigned v, unsigned* s
 
 // ---------------------------------------------------------------------------
 // Stable LSD radix sort, 9-bit digits (seven passes cover the 63-bit keys),
-// tiles of 4096 keys (512 threads x 8); three kernels per pass (tile
+// tiles of 4096 keys (512 threads x 8); two or three kernels per pass (tile
 // histograms, per-digit scans over the tiles, scatter)
 // ---------------------------------------------------------------------------
 
@@ -426,12 +426,17 @@ __global__ void __launch_bounds__(kRsThreads) rs_scan_kernel(unsigned* __restric
 constexpr size_t kRsScatterSmem = (size_t)kRsTile * (sizeof(unsigned long long) + sizeof(unsigned));
 static_assert(kRsWarps * kRsBins * sizeof(unsigned) <= kRsScatterSmem, "digit counters fit the tile buffer");
 
-__global__ void __launch_bounds__(kRsThreads, kRsScatterMinBlocks) rs_scatter_kernel(const unsigned long long* __restrict__ kin,
-                                                                const unsigned* __restrict__ vin,
-                                                                unsigned long long* __restrict__ kout,
-                                                                unsigned* __restrict__ vout, long long n, int shift,
-                                                                const unsigned* __restrict__ hist_scan,
-                                                                const unsigned* __restrict__ totals) {
+// FEW: the histogram is as rs_hist_kernel left it, and each thread adds its
+// digit's row up itself, which for few tiles is quicker than a launch of
+// rs_scan_kernel.
+template <bool FEW>
+__global__ void __launch_bounds__(kRsThreads, kRsScatterMinBlocks)
+    rs_scatter_kernel(const unsigned long long* __restrict__ kin,
+                      const unsigned* __restrict__ vin,
+                      unsigned long long* __restrict__ kout,
+                      unsigned* __restrict__ vout, long long n, int shift,
+                      const unsigned* __restrict__ hist_scan,
+                      const unsigned* __restrict__ totals) {
     extern __shared__ unsigned long long rs_smem[];
     unsigned long long* skeys = rs_smem;                             // kRsTile
     unsigned* svals = reinterpret_cast<unsigned*>(skeys + kRsTile);  // kRsTile
@@ -475,7 +480,7 @@ __global__ void __launch_bounds__(kRsThreads, kRsScatterMinBlocks) rs_scatter_ke
     // Per digit (thread t: digits kRsDpt t ...): exclusive prefix over warps
     // (stable: warp w precedes w+1), then over digits; the digit's global
     // offset is the scan of the digit totals plus this tile's row prefix.
-    unsigned run[kRsDpt], tot[kRsDpt];
+    unsigned run[kRsDpt], tot[kRsDpt], before[kRsDpt];
     unsigned rsum = 0, tsum = 0;
 #pragma unroll
     for (int j = 0; j < kRsDpt; ++j) {
@@ -487,7 +492,20 @@ __global__ void __launch_bounds__(kRsThreads, kRsScatterMinBlocks) rs_scatter_ke
             warp_cnt[ww][d] = run[j];
             run[j] += c;
         }
-        tot[j] = __ldg(totals + d);
+        if (FEW) {
+            const unsigned* row = hist_scan + d * gridDim.x;
+            tot[j] = 0;
+            before[j] = 0;
+#pragma unroll 8
+            for (unsigned b = 0; b < gridDim.x; ++b) {
+                const unsigned c = __ldg(row + b);
+                before[j] += b < blockIdx.x ? c : 0u;
+                tot[j] += c;
+            }
+        } else {
+            tot[j] = __ldg(totals + d);
+            before[j] = __ldg(hist_scan + d * gridDim.x + blockIdx.x);
+        }
         rsum += run[j];
         tsum += tot[j];
     }
@@ -498,7 +516,7 @@ __global__ void __launch_bounds__(kRsThreads, kRsScatterMinBlocks) rs_scatter_ke
     for (int j = 0; j < kRsDpt; ++j) {
         const unsigned d = kRsDpt * threadIdx.x + j;
         digit_start[d] = ds;
-        digit_base[d] = gs + hist_scan[d * gridDim.x + blockIdx.x];
+        digit_base[d] = gs + before[j];
         ds += run[j];
         gs += tot[j];
     }
@@ -537,7 +555,7 @@ __global__ void __launch_bounds__(kRsThreads, kRsScatterMinBlocks) rs_scatter_ke
 // 16 us a pass at any small size.  THREADS by size: the fewer warps, the
 // cheaper the prefix over them.  Sort phase (with the gather), before and now:
 // 1,000 bodies (2 passes) 37 and 15 us, 2,048 (3 passes) 64 and 19 us.  More keys
-// than one CTA holds keep three launches a pass (16,384 bodies: 78 us).
+// than one CTA holds take two or three launches a pass.
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS, 1) rs_single_kernel(unsigned long long* __restrict__ keys,
                                                               unsigned* __restrict__ vals, int n, int passes,
@@ -633,6 +651,9 @@ __global__ void __launch_bounds__(THREADS, 1) rs_single_kernel(unsigned long lon
 }
 
 constexpr int kRsSingleMax = 1024 * kRsItems;
+// Tiles up to which a pass is two launches (FEW): the sort of 16,384 bodies (4
+// tiles) takes 78 us with three and 63 with two, of 131,071 (32 tiles) 82 and 97.
+constexpr int kRsFewTiles = 12;
 
 template <int THREADS>
 static void launch_single(SortBuffers& sb, int n, int passes, int shift0, cudaStream_t s) {
@@ -658,9 +679,13 @@ int radix_sort_pairs(SortBuffers& sb, long long n, int passes, int shift0, cudaS
     const int nb = (int)((n + kRsTile - 1) / kRsTile);
     static bool attr_done = false;
     if (!attr_done) {
-        cudaFuncSetAttribute(rs_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRsScatterSmem);
+        cudaFuncSetAttribute(rs_scatter_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kRsScatterSmem);
+        cudaFuncSetAttribute(rs_scatter_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kRsScatterSmem);
         attr_done = true;
     }
+    const bool few = nb <= kRsFewTiles;
     unsigned* totals = sb.hist + (long long)nb * kRsBins;
     unsigned long long *kin = sb.keys, *kout = sb.keys_alt;
     unsigned *vin = sb.vals, *vout = sb.vals_alt;
@@ -671,12 +696,18 @@ int radix_sort_pairs(SortBuffers& sb, long long n, int passes, int shift0, cudaS
     for (int p = 0; p < passes; ++p) {
         const int shift = shift0 + kRsDigitBits * p;
         rs_hist_kernel<<<nb, kRsThreads, 0, s>>>(kin, n, shift, sb.hist);
-        rs_scan_kernel<<<kRsBins, kRsThreads, 0, s>>>(sb.hist, nb, totals);
-        rs_scatter_kernel<<<nb, kRsThreads, kRsScatterSmem, s>>>(kin, vin, kout, vout, n, shift, sb.hist, totals);
+        if (few) {
+            rs_scatter_kernel<true>
+                <<<nb, kRsThreads, kRsScatterSmem, s>>>(kin, vin, kout, vout, n, shift, sb.hist, totals);
+        } else {
+            rs_scan_kernel<<<kRsBins, kRsThreads, 0, s>>>(sb.hist, nb, totals);
+            rs_scatter_kernel<false>
+                <<<nb, kRsThreads, kRsScatterSmem, s>>>(kin, vin, kout, vout, n, shift, sb.hist, totals);
+        }
         std::swap(kin, kout);
         std::swap(vin, vout);
     }
-    return 3 * passes;
+    return (few ? 2 : 3) * passes;
 }
 
 // ---------------------------------------------------------------------------
