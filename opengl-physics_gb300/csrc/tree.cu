@@ -813,6 +813,7 @@ __global__ void __cluster_dims__(kTopCtas, 1, 1) __launch_bounds__(kTopThreads)
             look(l, node + kTopCtas * kTopThreads);
         }
         if (l > 0) look(l - 1, begin[l - 1] + tid);
+        __syncwarp();  // the loop's lanes leave it apart, and the barrier is .aligned
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
 }
