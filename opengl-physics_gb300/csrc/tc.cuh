@@ -46,8 +46,11 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
 }
 
 // Tensor memory: allocate / free `ncols` columns (a power of two >= 32) for
-// this CTA.  Executed by one full warp; the address lands in *slot.
+// this CTA.  Executed by one full warp; the address lands in *slot.  The warp
+// meets first, here and before the loads below: the instructions are .aligned,
+// and callers come out of one-thread branches and polling loops.
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)),
                  "r"(ncols)
                  : "memory");
@@ -55,6 +58,7 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {
 }
 
 __device__ __forceinline__ void tmem_free(uint32_t taddr, uint32_t ncols) {
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
@@ -112,6 +116,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity, uint3
 // thread i gets lane (taddr.lane + i), columns taddr.col .. +31.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float v[32]) {
     uint32_t r[32];
+    __syncwarp();
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
         "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"

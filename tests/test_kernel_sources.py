@@ -17,7 +17,7 @@ def statements(name):
     return [" ".join(s.split()) for s in re.split(r";(?=\s)(?!\\n)|(?<=[{}])\s", text) if s.strip()]
 
 
-@pytest.mark.parametrize("name", ["tree.cu"])
+@pytest.mark.parametrize("name", ["tree.cu", "tc.cuh"])
 def test_aligned_instructions_follow_a_reconvergence(name):
     """An .aligned instruction needs all threads of its warp at it together, so
     one comes directly after __syncwarp() (or after another of its kind)."""
