@@ -44,6 +44,12 @@ constexpr int kPpWarps = 4;
 constexpr int kPpThreads = kPpWarps * 32;
 constexpr int kPpTargets = 4;     // particles per slice: members walked together at most
 constexpr int kPpStack = 1024;    // union of the members' paths
+// Entries kept free for a walk that takes one node at a time: it leaves at most
+// seven siblings waiting per level.  Full up to here, the walk goes on so until
+// it is below again, and no tree outgrows the stack.  (A full stack cannot end
+// the walk: the slices done by then have had their closing kick.)  49,999 bodies
+// at leaf capacity 8, relative test, and substeps of 4,096: as fast as without.
+constexpr int kPpReserve = 7 * kMaxLevels;
 constexpr int kPpBuffer = 128;    // far nodes / near leaves waiting: 64 make a window or batch
 constexpr float kPpPad = 1e18f;   // position of the masked source that pads a window
 
@@ -351,12 +357,8 @@ __global__ void __launch_bounds__(kPpThreads, 4) walk_pp_kernel(NodeArrays T, Co
         PpWalk<SPLIT, QUAD, SOFT> w{sm, T, P, wp, lane, nt, {}};
         int nfar = 0, nnear = 0, visits = 0;
         while (size > 0) {
-            // at most eight children per node come back: never more than the stack holds
-            const int take = min(min(size, 32), (kPpStack - size) / 7);
-            if (take == 0) {
-                bad |= kStStackOverflow;
-                break;
-            }
+            // at most eight children per node come back
+            const int take = min(min(size, 32), max(1, (kPpStack - kPpReserve - size) / 7));
             size -= take;
             visits += take;
             if (visits > wp.node_limit) {
@@ -466,7 +468,7 @@ __global__ void __launch_bounds__(kPpThreads, 4) walk_pp_kernel(NodeArrays T, Co
                 nnear -= 64;
             }
         }
-        if (bad & (kStStackOverflow | kStCorrupt)) break;
+        if (bad) break;
         if (nfar > 0) w.far_window(nfar);
         if (nnear > 0) w.near_batch(nnear, own, active);
         // totals across the lanes, error-free but for the sum of the errors

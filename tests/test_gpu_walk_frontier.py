@@ -1,0 +1,80 @@
+"""Walks whose frontier outgrows their stack: trees in which a few cells of
+every level split and the rest wait, walked with nothing accepted.  Every
+particle then meets every other one, so accelerations equal the direct sum and
+steps the KDK step taken with it, whatever a walk does when its stack is full.
+Accelerations are held to the parity bars (median 1e-5, max 1e-4); a step's
+velocity change is a mean of two accelerations, so to the same."""
+import itertools
+
+import numpy as np
+import pytest
+
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+EPS, DT = 0.05, 1e-3
+OCTANTS = np.array(list(itertools.product((-1, 1), repeat=3)))[:, ::-1]  # x fastest, as in the keys
+
+
+def nest(width, levels, per_leaf=1):
+    """Positions in the lowest octant of the root cube, split once more into 64
+    cells; of these, and of the cells that come of it, the `width` last in key
+    order split into eight until there are `levels` levels below the octant.
+    Every other cell is left with `per_leaf` (1 or 2) particles, two in opposite
+    octants.  One particle more, at (1, 1, 1), holds the root cube."""
+    half = 0.5005  # of the root cube: the particles span 0 to 1
+    half /= 2
+    cells, left = [np.full(3, 0.5 - half)], []
+    for level in range(levels):
+        split = cells if level < 2 else cells[-width:]
+        left += [(c, half) for c in cells[:len(cells) - len(split)]]
+        half /= 2
+        cells = [c + half * o for c in split for o in OCTANTS]
+    left += [(c, half) for c in cells]
+    inside = (OCTANTS[0], OCTANTS[7]) if per_leaf == 2 else (0 * OCTANTS[0],)
+    p = np.array([c + h / 2 * o for c, h in left for o in inside] + [np.ones(3)])
+    p[np.argmin(p.sum(1))] = 0.0
+    return p.T.copy(), np.random.default_rng(levels).uniform(0.5, 1.5, len(p)) / len(p)
+
+
+def direct(x, m):
+    a = np.empty_like(x)
+    for i in range(x.shape[1]):
+        d = x - x[:, i:i + 1]
+        a[:, i] = (m * ((d * d).sum(0) + EPS ** 2) ** -1.5 * d).sum(1)
+    return a
+
+
+def bars(a, want):
+    e = rel_err(*a, *want)
+    assert np.median(e) <= 1e-5 and e.max() <= 1e-4, (np.median(e), e.max())
+
+
+def system(pkg, x, m, theta=0.0, **kw):
+    sim = pkg.NBodySystem(pkg.StepParams(G=1.0, eps=EPS, theta=theta), leaf_capacity=1, **kw)
+    sim.set_particles(*x, None, None, None, m.astype(np.float32).astype(np.float64))
+    return sim
+
+
+@pytest.mark.parametrize("kind", ["relative", "block"])
+@pytest.mark.parametrize("width,levels", [(32, 3), (32, 8), (40, 19)])
+def test_per_particle_walk(pkg, kind, width, levels):
+    """At 8 levels and at 19 more than the 1,024 nodes that a walk keeps would wait."""
+    x, m = nest(width, levels)
+    with system(pkg, x, m, mac=pkg.MAC_RELATIVE if kind == "relative" else pkg.MAC_GEOMETRIC) as sim:
+        if kind == "relative":
+            sim.set_mac_alpha(1e-30)  # the relative test accepts nothing either
+        sim.prime()
+        m = m.astype(np.float32).astype(np.float64)
+        a0 = direct(x, m)
+        bars(sim.accel(), a0)
+        if kind == "relative":
+            sim.step(1, DT)
+        else:
+            sim.block_step(DT, eta=1e3, max_rung=0)
+        st = sim.stats()
+        assert st["p2p_pairs"] == len(m) * (len(m) - 1) and st["p2c_terms"] == 0
+        a1 = direct(x + DT * (0.5 * DT * a0), m)
+        bars(sim.accel(), a1)
+        bars(np.array(sim.state()[3:6]) / DT, 0.5 * (a0 + a1))
