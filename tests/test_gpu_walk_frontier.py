@@ -78,3 +78,39 @@ def test_per_particle_walk(pkg, kind, width, levels):
         a1 = direct(x + DT * (0.5 * DT * a0), m)
         bars(sim.accel(), a1)
         bars(np.array(sim.state()[3:6]) / DT, 0.5 * (a0 + a1))
+
+
+@pytest.mark.parametrize("learned", [False, True])
+@pytest.mark.parametrize("stack,levels", [(1024, 8), (2048, 14)])
+def test_grouped_walk_leaves_shared_memory(pkg, learned, stack, levels):
+    """stack / 4 opened nodes fit in shared memory; these trees have more."""
+    x, m = nest(8, levels, per_leaf=2)
+    with system(pkg, x, m) as sim:
+        sim.set_tuning(p2p_tile=0, walk_stack=stack)
+        if learned:
+            open_everything(pkg, sim, rho_hi=1e-6)
+        bars(sim.compute_accel(), direct(x, m.astype(np.float32).astype(np.float64)))
+        st = sim.stats()
+    assert st["walk_stack_max"] > stack
+    assert st["p2p_pairs"] == len(m) * (len(m) - 1) and st["p2c_terms"] == 0
+
+
+def open_everything(pkg, sim, **opts):
+    """The learned walk with a network that never decides (the geometric test
+    does) and a band that starts at rho_lo = 0."""
+    sim.lmac_set_model(np.zeros(1377, np.float32), np.ones(16, np.float32))
+    sim.lmac_set_opts(gate=1e30, rho_lo=0.0, check_every=0, screen=0.0, **opts)
+    sim.prime()  # the learned test reads accelerations
+    sim.set_opts(mac=pkg.MAC_LEARNED)
+
+
+def test_learned_walk_outgrows_the_global_stack(pkg):
+    """A round that opens 4,096 nodes at once: the global-memory stack, 2,048
+    opened nodes at first, is doubled."""
+    x, m = nest(4096, 4, per_leaf=2)  # all 4,096 cells of a level split
+    with system(pkg, x, m) as sim:
+        open_everything(pkg, sim, rho_hi=1e30, rounds=8)
+        bars(sim.compute_accel(), direct(x, m.astype(np.float32).astype(np.float64)))
+        st = sim.stats()
+    assert st["walk_stack_max"] > 4 * 2048
+    assert st["p2p_pairs"] == len(m) * (len(m) - 1) and st["p2c_terms"] == 0
