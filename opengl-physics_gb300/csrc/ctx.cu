@@ -956,10 +956,7 @@ int ngrav_gpu_diagnostics(ngrav_gpu_ctx* ctx, int exact_potential, ngrav_gpu_dia
         for (int b = 0; b < pb; ++b) pot += hp[b];
         out->potential = ctx->opts.G * pot;
     } else if (exact) {
-        const double mscale =
-            potential_scaled(n) && std::isfinite(M) && M != 0.0 ? std::ldexp(1.0, -std::ilogb(M)) : 1.0;
-        launch_potential(n, ctx->P, split, ctx->opts.eps * ctx->opts.eps, spline_h(ctx), mscale, ctx->dpartial,
-                         ctx->stream);
+        launch_potential(n, ctx->P, split, ctx->opts.eps * ctx->opts.eps, spline_h(ctx), ctx->dpartial, ctx->stream);
         NG_CUDA(cudaMemcpyAsync(h.data(), ctx->dpartial, sizeof(double) * npb, cudaMemcpyDeviceToHost,
                                 ctx->stream));
         NG_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -971,7 +968,7 @@ int ngrav_gpu_diagnostics(ngrav_gpu_ctx* ctx, int exact_potential, ngrav_gpu_dia
             pot = t;
         }
         if (std::isfinite(low)) pot += low;
-        out->potential = ctx->opts.G * (pot / mscale / mscale);
+        out->potential = ctx->opts.G * pot;
     } else {
         out->potential = std::nan("");
     }

@@ -22,17 +22,14 @@ int diag_blocks(long long n);
 void launch_diag_pass1(long long n, const Particles& P, bool split, double* partial, cudaStream_t s);
 void launch_diag_pass2(long long n, const Particles& P, bool split, double cx, double cy, double cz, double* partial,
                        cudaStream_t s);
-// potential.cu: the exact pair potential, one partial sum per block.  Where
-// potential_scaled(n), every mass is taken times mscale, a power of two near
-// 1 / (total mass): the sum is then mscale^2 times the potential.
+// potential.cu: the exact pair potential, one partial sum per block.
 int potential_blocks(long long n);
-bool potential_scaled(long long n);
 // Exact pair potential with FP32 pair terms and FP64 sums (Plummer).
 int potential_f32_blocks(long long n, int sm_count);
 void launch_potential_f32(long long n, const Particles& P, bool split, double eps2, int blocks, double* partial,
                           cudaStream_t s);
-void launch_potential(long long n, const Particles& P, bool split, double eps2, double spline_h, double mscale,
-                      double* partial, cudaStream_t s);
+void launch_potential(long long n, const Particles& P, bool split, double eps2, double spline_h, double* partial,
+                      cudaStream_t s);
 int sampler_shares(long long n, int nslots, int sm_count);
 // FP64 pairs (one block per target), or FP32 pairs tiled over `shares`
 // source shares with FP64 totals (partial: shares * 3 * nslots doubles).

@@ -199,7 +199,8 @@ __device__ __noinline__ PotPair refine_pair(float4 th, float4 tl, float4 qh, flo
 struct __align__(16) PotStage {
     float x1[3][kPotThreads];  // source coordinates in the frame: grid part
     float x2[3][kPotThreads];  //   and the rest
-    float m[kPotThreads];      // mass x mscale x frame scale
+    float m[kPotThreads];      // masses, the frame's largest in [1, 2)
+    double unit[kPotThreads / kPotSub];        // what a sum in the frame's units is worth
     float sc[kPotThreads / kPotSub], e2h[kPotThreads / kPotSub], e2l[kPotThreads / kPotSub],
         near2[kPotThreads / kPotSub], kernel2[kPotThreads / kPotSub];
 };
@@ -236,7 +237,7 @@ __device__ __forceinline__ double pot_block_sum(double v) {
 template <bool SPLIT>
 __global__ void __launch_bounds__(kPotThreads, 5) potential_df_kernel(long long n, const float4* __restrict__ pos,
                                                                       const float4* __restrict__ plo, double eps2,
-                                                                      double spline_h, double mscale, long long chunk,
+                                                                      double spline_h, long long chunk,
                                                                       double* __restrict__ partial) {
     __shared__ PotStage sm;
     __shared__ unsigned s_rho;
@@ -290,7 +291,12 @@ __global__ void __launch_bounds__(kPotThreads, 5) potential_df_kernel(long long 
             // range (or a NaN) sends every pair of the frame to refine_pair,
             // and from there to FP64
             const unsigned eb = a >> 23;
-            const bool fits = eb >= 8u && eb <= 245u;
+            // and so does a source lighter than 2^-63 of the heaviest: its low
+            // parts (2^-46 of its term) would not be normal numbers
+            const unsigned mb = __float_as_uint(fabsf(q.w));
+            const unsigned heaviest = __reduce_max_sync(0xffffffffu, mb) >> 23;
+            const unsigned lightest = __reduce_min_sync(0xffffffffu, mb ? mb : 0xffffffffu) >> 23;
+            const bool fits = eb >= 8u && eb <= 245u && lightest > 0u && lightest + 63u >= heaviest && heaviest < 255u;
             const float sc = fits ? __uint_as_float((253u - eb) << 23) : 1.f;
             const double scd = (double)sc, e2 = spline_h > 0.0 || !fits ? 0.0 : eps2 * scd * scd;
 #pragma unroll
@@ -300,8 +306,10 @@ __global__ void __launch_bounds__(kPotThreads, 5) potential_df_kernel(long long 
                 sm.x1[k][tid] = fits ? x1 : 0.f;
                 sm.x2[k][tid] = fits ? x2 : 0.f;
             }
-            sm.m[tid] = (float)((double)q.w * mscale * scd);
+            // in units of 2^(heaviest - 127)
+            sm.m[tid] = fits ? (float)((double)q.w * __longlong_as_double((long long)(1150u - heaviest) << 52)) : 0.f;
             if (lane == 0) {
+                sm.unit[w] = __longlong_as_double((long long)(896u + heaviest) << 52) * scd;
                 const float inf = __uint_as_float(0x7f800000u);
                 // rounded up, so that every pair inside the kernel is caught
                 const float k2 = spline_h > 0.0 ? (float)(4.00001 * (spline_h * scd) * (spline_h * scd)) : 0.f;
@@ -364,7 +372,7 @@ __global__ void __launch_bounds__(kPotThreads, 5) potential_df_kernel(long long 
                                                               sm.kernel2[f], eps2, spline_h);
                                 y = p.y;
                                 co = p.corr;
-                                acc += (double)qh.w * mscale * p.wide;
+                                acc += (double)qh.w * p.wide;
                             }
                             if (u) {
                                 y0.y = y;
@@ -387,11 +395,11 @@ __global__ void __launch_bounds__(kPotThreads, 5) potential_df_kernel(long long 
             }
             float S, er;
             sum2(A.x, A.y, S, er);
-            acc += (double)S;
-            acc += (double)(er + (R.x + R.y));
+            acc = fma((double)S, sm.unit[f], acc);
+            acc = fma((double)(er + (R.x + R.y)), sm.unit[f], acc);
         }
     }
-    const double t = pot_block_sum(have ? -(double)th.w * mscale * acc : 0.0);
+    const double t = pot_block_sum(have ? -(double)th.w * acc : 0.0);
     if (tid == 0) *out = t;
 }
 
@@ -440,20 +448,17 @@ __global__ void __launch_bounds__(kPotThreads) potential_f64_kernel(long long n,
     if (tid == 0) *out = t;
 }
 
-bool potential_scaled(long long n) { return n >= kPotDfMin; }
-
-void launch_potential(long long n, const Particles& P, bool split, double eps2, double spline_h, double mscale,
-                      double* partial, cudaStream_t s) {
+void launch_potential(long long n, const Particles& P, bool split, double eps2, double spline_h, double* partial,
+                      cudaStream_t s) {
     const dim3 grid((unsigned)pot_tiles(n), (unsigned)pot_chunks(n));
     const long long chunk = potential_chunk(n);
-    if (!potential_scaled(n))
+    if (n < kPotDfMin)
         potential_f64_kernel<<<grid, kPotThreads, 0, s>>>(n, P.pos, split ? P.plo : nullptr, eps2, spline_h, chunk,
                                                           partial);
     else if (split)
-        potential_df_kernel<true><<<grid, kPotThreads, 0, s>>>(n, P.pos, P.plo, eps2, spline_h, mscale, chunk, partial);
+        potential_df_kernel<true><<<grid, kPotThreads, 0, s>>>(n, P.pos, P.plo, eps2, spline_h, chunk, partial);
     else
-        potential_df_kernel<false><<<grid, kPotThreads, 0, s>>>(n, P.pos, nullptr, eps2, spline_h, mscale, chunk,
-                                                                partial);
+        potential_df_kernel<false><<<grid, kPotThreads, 0, s>>>(n, P.pos, nullptr, eps2, spline_h, chunk, partial);
 }
 
 }  // namespace ngrav

@@ -1,0 +1,47 @@
+"""The exact pair potential where masses, lengths or single pairs are far from
+the rest: light particles round a heavy one in large units, coordinates at the
+ends of FP32's range, a few pairs that carry the energy.  Compared with an FP64
+pair sum (numpy, compensated over the rows) of the same float32 masses and
+double-float positions.
+
+Tolerance: 1e-14 of the sum.  An FP64 term is good to a few 2^-53 (the
+reference's too) and both sides add up 10^7 terms of one sign per thousands of
+partial sums: 1e-15 with room."""
+import numpy as np
+import pytest
+
+from test_gpu_potential import pair_sum
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-14
+
+
+def check(pkg, x, y, z, m, eps, spline=False, sort=False, precision=1, tol=TOL):
+    with pkg.NBodySystem(pkg.StepParams(G=1.0, eps=eps, theta=0.6), leaf_capacity=16, precision=precision) as sim:
+        if spline:
+            sim.set_softening(pkg.SOFTENING_SPLINE)
+        sim.set_particles(x, y, z, None, None, None, m)
+        if sort:
+            sim.prime()
+        got = sim.diagnostics(exact_potential=1)
+        st = sim.state()
+    want = pair_sum(*st[:3], np.asarray(m, np.float32).astype(np.float64), eps, spline)
+    assert got["potential_exact"] == 1 and np.isfinite(want)
+    assert abs(got["potential"] - want) <= tol * abs(want), (got["potential"], want)
+
+
+def plummer(ic, n, seed=4):
+    x, y, z, _, _, _, _ = ic.plummer(n, seed=seed)
+    return [np.float64(a) for a in (x, y, z)]
+
+
+@pytest.mark.parametrize("at", [0, 40, 2600, 4999])
+@pytest.mark.parametrize("length,heavy,light", [(1e9, 1.0, 1e-30), (5e11, 2e30, 1.0), (1e-9, 1e-3, 1e-33), (1.0, 1.0, 1e-37)])
+def test_heavy_body_and_tracers(pkg, ic, length, heavy, light, at):
+    """Tracers down to 1e-37 of the heavy body's mass, which is the first, one of
+    the first or the last in the order of the pairs."""
+    x, y, z = (a * length for a in plummer(ic, 5000))
+    m = np.full(5000, light) * np.random.default_rng(1).uniform(0.5, 1.5, 5000)
+    m[at] = heavy
+    check(pkg, x, y, z, m, 0.01 * length)
