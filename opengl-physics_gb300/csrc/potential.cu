@@ -152,6 +152,22 @@ __device__ __forceinline__ double pair_phi(double dx, double dy, double dz, doub
     return rsqrt(dx * dx + dy * dy + dz * dz + eps2);
 }
 
+// The sources [jf, j_end) after target i, in FP64: of a frame whose numbers FP32
+// does not hold.
+__device__ __noinline__ double frame_f64(const float4* __restrict__ pos, const float4* __restrict__ plo, float4 th,
+                                         float4 tl, long long i, long long jf, long long j_end, double eps2,
+                                         double spline_h) {
+    const double x = (double)th.x + (double)tl.x, y = (double)th.y + (double)tl.y, z = (double)th.z + (double)tl.z;
+    double sum = 0.0;
+    for (long long j = jf > i ? jf : i + 1; j < j_end; ++j) {
+        const float4 q = pos[j];
+        const float4 l = plo ? plo[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+        sum += (double)q.w * pair_phi(((double)q.x + (double)l.x) - x, ((double)q.y + (double)l.y) - y,
+                                      ((double)q.z + (double)l.z) - z, eps2, spline_h);
+    }
+    return sum;
+}
+
 struct PotPair {
     float y, corr;  // double-float 1/r in the frame's unit (0, 0 when `wide` holds the term)
     double wide;    // 1/r or the spline's -phi/h in FP64, in the caller's unit
@@ -200,7 +216,7 @@ struct __align__(16) PotStage {
     float x1[3][kPotThreads];  // source coordinates in the frame: grid part
     float x2[3][kPotThreads];  //   and the rest
     float m[kPotThreads];      // masses, the frame's largest in [1, 2)
-    double unit[kPotThreads / kPotSub];        // what a sum in the frame's units is worth
+    double unit[kPotThreads / kPotSub];        // what a sum in the frame's units is worth (0: summed in FP64)
     float sc[kPotThreads / kPotSub], e2h[kPotThreads / kPotSub], e2l[kPotThreads / kPotSub],
         near2[kPotThreads / kPotSub], kernel2[kPotThreads / kPotSub];
 };
@@ -287,42 +303,46 @@ __global__ void __launch_bounds__(kPotThreads, 5) potential_df_kernel(long long 
             unsigned a = max(max(__float_as_uint(fabsf(yh[0])), __float_as_uint(fabsf(yh[1]))),
                              __float_as_uint(fabsf(yh[2])));
             a = max(__reduce_max_sync(0xffffffffu, a), s_rho);
-            // 2^-ex with E = 2^ex [1/2, 1); an E outside FP32's comfortable
-            // range (or a NaN) sends every pair of the frame to refine_pair,
-            // and from there to FP64
+            // 2^-ex with E = 2^ex [1/2, 1).  A frame is summed in FP64 if E is
+            // outside FP32's comfortable range (or a NaN), or if a source is
+            // lighter than 2^-63 of the heaviest: its low parts (2^-46 of its
+            // term) would not be normal numbers.
             const unsigned eb = a >> 23;
-            // and so does a source lighter than 2^-63 of the heaviest: its low
-            // parts (2^-46 of its term) would not be normal numbers
             const unsigned mb = __float_as_uint(fabsf(q.w));
             const unsigned heaviest = __reduce_max_sync(0xffffffffu, mb) >> 23;
             const unsigned lightest = __reduce_min_sync(0xffffffffu, mb ? mb : 0xffffffffu) >> 23;
             const bool fits = eb >= 8u && eb <= 245u && lightest > 0u && lightest + 63u >= heaviest && heaviest < 255u;
             const float sc = fits ? __uint_as_float((253u - eb) << 23) : 1.f;
-            const double scd = (double)sc, e2 = spline_h > 0.0 || !fits ? 0.0 : eps2 * scd * scd;
+            const double scd = (double)sc, e2 = spline_h > 0.0 ? 0.0 : eps2 * scd * scd;
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 float x1, x2;
                 grid_split(yh[k], yl[k], sc, x1, x2);
-                sm.x1[k][tid] = fits ? x1 : 0.f;
-                sm.x2[k][tid] = fits ? x2 : 0.f;
+                sm.x1[k][tid] = x1;
+                sm.x2[k][tid] = x2;
             }
             // in units of 2^(heaviest - 127)
-            sm.m[tid] = fits ? (float)((double)q.w * __longlong_as_double((long long)(1150u - heaviest) << 52)) : 0.f;
+            sm.m[tid] = (float)((double)q.w * __longlong_as_double((long long)(1150u - heaviest) << 52));
             if (lane == 0) {
-                sm.unit[w] = __longlong_as_double((long long)(896u + heaviest) << 52) * scd;
-                const float inf = __uint_as_float(0x7f800000u);
+                sm.unit[w] = fits ? __longlong_as_double((long long)(896u + heaviest) << 52) * scd : 0.0;
                 // rounded up, so that every pair inside the kernel is caught
                 const float k2 = spline_h > 0.0 ? (float)(4.00001 * (spline_h * scd) * (spline_h * scd)) : 0.f;
                 sm.sc[w] = sc;
                 sm.e2h[w] = (float)e2;
                 sm.e2l[w] = (float)(e2 - (double)(float)e2);
-                sm.kernel2[w] = fits ? k2 : inf;
-                sm.near2[w] = fits ? fmaxf(kPotNear2, k2) : inf;
+                sm.kernel2[w] = k2;
+                sm.near2[w] = fmaxf(kPotNear2, k2);
             }
         }
         __syncthreads();
         const int frames = (int)((min((long long)kPotThreads, j_end - t) + kPotSub - 1) / kPotSub);
         for (int f = 0; f < frames; ++f) {
+            const long long jf = t + f * kPotSub;
+            const double unit = sm.unit[f];
+            if (unit == 0.0) {
+                if (have) acc += frame_f64(pos, SPLIT ? plo : nullptr, th, tl, i, jf, min(jf + kPotSub, j_end), eps2, spline_h);
+                continue;
+            }
             const float sc = sm.sc[f], near2 = sm.near2[f];
             const float2 e2h = splat<float2>(sm.e2h[f]), e2l = splat<float2>(sm.e2l[f]);
             float2 n1[3], n2[3];  // the target, negated
@@ -333,7 +353,6 @@ __global__ void __launch_bounds__(kPotThreads, 5) potential_df_kernel(long long 
                 n1[k] = splat<float2>(-x1);
                 n2[k] = splat<float2>(-x2);
             }
-            const long long jf = t + f * kPotSub;
             const bool diag = jf < i0 + kPotThreads;  // sources at or before some target
             float2 A = make_float2(0.f, 0.f), R = A;
             for (int k4 = 0; k4 < kPotSub; k4 += 4) {
@@ -395,8 +414,8 @@ __global__ void __launch_bounds__(kPotThreads, 5) potential_df_kernel(long long 
             }
             float S, er;
             sum2(A.x, A.y, S, er);
-            acc = fma((double)S, sm.unit[f], acc);
-            acc = fma((double)(er + (R.x + R.y)), sm.unit[f], acc);
+            acc = fma((double)S, unit, acc);
+            acc = fma((double)(er + (R.x + R.y)), unit, acc);
         }
     }
     const double t = pot_block_sum(have ? -(double)th.w * acc : 0.0);

@@ -45,3 +45,11 @@ def test_heavy_body_and_tracers(pkg, ic, length, heavy, light, at):
     m = np.full(5000, light) * np.random.default_rng(1).uniform(0.5, 1.5, 5000)
     m[at] = heavy
     check(pkg, x, y, z, m, 0.01 * length)
+
+
+@pytest.mark.parametrize("spline", [False, True])
+@pytest.mark.parametrize("length", [1e30, 1e36, 1.5e37])
+def test_extent_near_the_end_of_fp32(pkg, ic, length, spline):
+    """Squares of the distances are past FP32's range, at 1.5e37 some differences too."""
+    x, y, z = (a * length for a in plummer(ic, 5000))
+    check(pkg, x, y, z, np.full(5000, 1.0 / 5000), 0.01 * length, spline)
