@@ -2,39 +2,48 @@
 // sum over i < j of -m_i m_j / sqrt(r^2 + eps^2) (Plummer) or m_i m_j phi(r/h)/h
 // (spline), restating System::TotalEnergy (include/ngrav/System.hpp:119-150).
 //
-// Every pair term is needed to double-precision accuracy, and GB300's FP64
-// pipe runs at 1/64 of the FP32 rate: an FP64 pair costs about 21 FP64
-// operations, 1,344 FP32 slots.  potential_df_kernel forms each term on the
-// packed FP32 pipe as an unevaluated pair of floats instead, in about 52 FP32
-// operations, and leaves FP64 to the sums (one flush per 32 sources):
+// The sum is needed to double-precision accuracy, and GB300's FP64 pipe runs at
+// 1/64 of the FP32 rate: an FP64 pair costs about 21 FP64 operations, 1,344 FP32
+// slots.  potential_df_kernel forms each term on the packed FP32 pipe as an
+// unevaluated pair of floats instead, in about 54 FP32 operations, and leaves
+// FP64 to the sums (one flush per 32 sources):
 //
 //  * Frame.  Targets and sources of a (128 targets, 32 sources) tile are taken
 //    relative to the tile's middle target and scaled by a power of two so the
 //    largest |coordinate| E lies in [1/2, 1).  Each coordinate is split into
 //    x1 on the grid 2^-22 and the rest x2, so a difference of two x1 is exact
 //    in one subtraction and the difference of two x2 is off by 2^-48 E only.
+//    Masses are scaled by a power of two so the largest of the 32 lies in [1, 2).
 //  * r^2 + eps^2.  B = the FP32 sum of squares seeds three fused steps h += s^2
 //    that all round at B's exponent; h_k - h_(k-1) is then exact (Sterbenz) and
 //    one more fma recovers what each step rounded off, so B plus the collected
-//    remainder is r^2 + eps^2 to about 2^-46.
+//    remainder is r^2 + eps^2 (inv_dist).
 //  * 1/r.  The hardware reciprocal square root y0 of B, with the residual
 //    e = 1 - (r^2 + eps^2) y0^2 taken by fma: y = y0 (1 + e/2 + 3/8 e^2).
 //  * Sum.  m y0 + m corr as a float pair, two-sum accumulated over 32 sources,
 //    then added to the thread's FP64 total.
 //
-// The x2 differences limit close pairs (E / r x 2^-47), so a pair nearer than
-// E/16 is formed again from the particles' own double-float positions with
-// error-free differences (refine_pair), and pairs inside the spline's kernel,
-// at r = 0 or outside FP32's range take the FP64 formula.  Emulated on the
-// CPU with exact rounding against 80-bit sums (Plummer spheres, eps 0 to
-// 0.05): the sum's relative error at n >= 4,096 is 1e-16 to 5e-16, the same
-// as with FP64 terms (1e-16 to 8e-16); at n = 1,000 it is 1e-15 against 1e-16
-// (too few terms to average over), hence kPotDfMin.
+// What a term is good to falls with its distance, as the remainder and the
+// differences of the x2 are single FP32 numbers: rms 2^-46 of it at r = E, 2^-42 at
+// E/16, 2^-38.8 at worst.  So a sum is as good as its terms are many and their
+// errors independent, and the rest goes other ways:
+//  * a pair nearer than E/16 is formed again from the particles' own double-float
+//    positions with error-free differences (refine_pair), and pairs inside the
+//    spline's kernel or at r = 0 take the FP64 formula;
+//  * 32 sources whose numbers FP32 does not hold are summed in FP64 (frame_f64),
+//    and so are all pairs below kPotDfMin.
+// Emulated on the CPU with exact rounding against 80-bit sums (Plummer spheres in
+// double-float and in FP32 positions, eps 0 to 0.05), the sum's relative error, rms
+// and worst, and that of FP64 terms: n = 1,000 6e-16, 1e-15 and 2e-16, 4e-16; 2,048
+// 4e-16, 6e-16 and 2e-16, 4e-16; 4,096 1e-16, 2e-16 and 3e-16, 5e-16; 16,384 5e-17,
+// 1e-16 and 4e-16, 7e-16; hence kPotDfMin.  On the GPU, 4,096 to 16,384 bodies
+// (Plummer, galaxy; both softenings): rms 7e-17, worst 1.9e-16 in tree order, 2e-16
+// and 3.6e-16 in another; FP64 terms 1.8e-16 and 5.7e-16.
 //
 // Measured (GB300, one diagnostics call on a Plummer sphere in tree order):
-// 131,071 particles 299 ms with FP64 terms -> 17.1 ms (0.70 of the FP32 pipe's
-// 52-operation time), 16,384 15.0 -> 0.35 ms, 2,048 (FP64 blocks of 32 sources
-// instead of whole rows) 1.87 -> 0.17 ms; spline, 20,011: 53.6 -> 0.66 ms.
+// 131,071 particles 299 ms with FP64 terms -> 18.0 ms (0.69 of the FP32 pipe's
+// 54-operation time), 16,384 15.0 -> 0.37 ms, 2,048 (FP64 blocks of 32 sources
+// instead of whole rows) 1.87 -> 0.17 ms; spline, 20,011: 53.6 -> 0.7 ms.
 // Particles not yet in tree order have wide frames, so more pairs take
 // refine_pair: 45 ms at 131,071.
 #include "ctx_kernels.cuh"
@@ -49,8 +58,8 @@ constexpr int kPotThreads = 128;           // targets per block
 constexpr int kPotSub = 32;                // sources per frame (one staging warp)
 constexpr int kPotChunkMax = 8192;         // sources per block at most, but no more than
 constexpr int kPotChunks = 16;             //   this many blocks per target tile
-// Smallest n of the double-float kernel.  Below it FP64 terms are exact to
-// the last bit of the sum and cheap (4,095: 8.4 M pairs).
+// Smallest n of the double-float kernel: from here on its error is below that of
+// FP64 terms (above); 4,095 particles in FP64 take as long as 16,384 without.
 constexpr long long kPotDfMin = 4096;
 constexpr float kPotNear2 = 1.f / 512.f;   // (E/16)^2 at E = 1/sqrt(2); E is in [1/2, 1)
 
@@ -103,15 +112,13 @@ __device__ __forceinline__ void sum2(V a, V b, V& s, V& e) {
     e = vadd(vsub(a, vsub(s, bb)), vsub(b, bb));
 }
 
-// What one fused step h += s^2 rounded off, plus l (2 s + l): the axis's
-// share of r^2 that the running sum does not hold.  `h` moves on.
+// One fused step h += s^2; returns what it rounded off.
 template <class V>
-__device__ __forceinline__ V square_step(V s, V l, V& h) {
+__device__ __forceinline__ V square_step(V s, V& h) {
     const V h2 = vfma(s, s, h);
-    const V nd = vsub(h, h2);
-    const V f = vfma(vfma(splat<V>(2.f), s, l), l, vfma(s, s, nd));
+    const V rest = vfma(s, s, vsub(h, h2));
     h = h2;
-    return f;
+    return rest;
 }
 
 // B: FP32 r^2 + eps^2 from the leading differences.
@@ -120,23 +127,35 @@ __device__ __forceinline__ V lead_r2(const V s[3], V e2h) {
     return vfma(s[0], s[0], vfma(s[1], s[1], vfma(s[2], s[2], e2h)));
 }
 
-// 1 / sqrt(|s + l|^2 + eps^2) as y0 + corr, B = lead_r2(s); ny0 = -y0.
+// 1 / sqrt(|s + l|^2 + eps^2) as y0 + corr, from l2 = 2 l and B = lead_r2(s);
+// ny0 = -y0.
+//
+// No rounding here may lean one way, or millions of terms add it up: 2^-50 of
+// each would be more than the error of an FP64 sum.  So
+//  * the cross terms are fused products s l2, exact before they are rounded, and
+//    what the square steps rounded off and the error of adding e2h (all on the
+//    grid 2^-44) are added exactly: a constant of finer bits would be rounded the
+//    same way in every pair of a frame;
+//  * what is always positive, |l|^2 and the rest of eps^2, comes in under a fused
+//    product with y0, whose low bits differ from pair to pair;
+//  * the second-order term of corr (3/8 e^2, about 2^-47) is added to e, and not
+//    to 1/2, whose grid would swallow it.
 template <class V>
-__device__ __forceinline__ void inv_dist(const V s[3], const V l[3], V e2h, V e2l, V B, V& y0, V& ny0, V& corr) {
+__device__ __forceinline__ void inv_dist(const V s[3], const V l2[3], V e2h, V e2l, V B, V& y0, V& ny0, V& corr) {
     y0 = vrsqrt(B);
     ny0 = vneg(y0);
     V h = B;
-    const V f0 = square_step(s[0], l[0], h);
-    const V f1 = square_step(s[1], l[1], h);
-    const V f2 = square_step(s[2], l[2], h);
+    const V r0 = square_step(s[0], h), r1 = square_step(s[1], h), r2 = square_step(s[2], h);
     const V h4 = vadd(h, e2h);
-    const V f3 = vadd(vadd(e2h, vsub(h, h4)), e2l);
-    const V rest = vadd(vadd(f0, f1), vadd(f2, f3));
-    const V low = vadd(vfma(splat<V>(-2.f), B, h4), rest);  // r^2 + eps^2 - B
+    const V p = vadd(e2h, vsub(h, h4));
+    const V rest = vadd(vadd(r0, r1), vadd(r2, vfma(splat<V>(-2.f), B, h4)));
+    const V low = vadd(rest, vfma(s[2], l2[2], vfma(s[1], l2[1], vfma(s[0], l2[0], p))));
+    const V ll = vfma(l2[0], l2[0], vfma(l2[1], l2[1], vmul(l2[2], l2[2])));
+    const V least = vfma(splat<V>(0.25f), ll, e2l);  // B + low + least = r^2 + eps^2
     const V nz = vmul(B, ny0);
-    const V v = vfma(low, y0, vfma(B, y0, nz));
+    const V v = vfma(low, y0, vfma(least, y0, vfma(B, y0, nz)));
     const V e = vfma(v, ny0, vfma(nz, y0, splat<V>(1.f)));
-    corr = vmul(y0, vmul(e, vfma(splat<V>(0.375f), e, splat<V>(0.5f))));
+    corr = vmul(vmul(splat<V>(0.5f), y0), vfma(vmul(splat<V>(0.75f), e), e, e));
 }
 
 // ---------------------------------------------------------------------------
@@ -180,7 +199,7 @@ __device__ __noinline__ PotPair refine_pair(float4 th, float4 tl, float4 qh, flo
                                             float e2l, float kernel2, double eps2, double spline_h) {
     const float a[3] = {qh.x, qh.y, qh.z}, al[3] = {ql.x, ql.y, ql.z};
     const float b[3] = {th.x, th.y, th.z}, bl[3] = {tl.x, tl.y, tl.z};
-    float s[3], l[3];
+    float s[3], l2[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         float d, de, q, qe, u, ue;
@@ -190,7 +209,7 @@ __device__ __noinline__ PotPair refine_pair(float4 th, float4 tl, float4 qh, flo
         float hi, lo;
         sum2(d, u, hi, lo);
         s[k] = hi * sc;
-        l[k] = (lo + (qe + ue)) * sc;
+        l2[k] = 2.f * ((lo + (qe + ue)) * sc);
     }
     const float B = lead_r2(s, e2h);
     PotPair r = {0.f, 0.f, 0.0};
@@ -198,7 +217,7 @@ __device__ __noinline__ PotPair refine_pair(float4 th, float4 tl, float4 qh, flo
     // ends of its range (a NaN fails both)
     if (B >= kernel2 && B >= 1e-20f && B <= 16.f) {
         float ny;
-        inv_dist(s, l, e2h, e2l, B, r.y, ny, r.corr);
+        inv_dist(s, l2, e2h, e2l, B, r.y, ny, r.corr);
         return r;
     }
     const double dx = ((double)qh.x + (double)ql.x) - ((double)th.x + (double)tl.x);
@@ -214,7 +233,7 @@ __device__ __noinline__ PotPair refine_pair(float4 th, float4 tl, float4 qh, flo
 
 struct __align__(16) PotStage {
     float x1[3][kPotThreads];  // source coordinates in the frame: grid part
-    float x2[3][kPotThreads];  //   and the rest
+    float x2[3][kPotThreads];  //   and twice the rest
     float m[kPotThreads];      // masses, the frame's largest in [1, 2)
     double unit[kPotThreads / kPotSub];        // what a sum in the frame's units is worth (0: summed in FP64)
     float sc[kPotThreads / kPotSub], e2h[kPotThreads / kPotSub], e2l[kPotThreads / kPotSub],
@@ -230,10 +249,10 @@ __device__ __forceinline__ void rel_coord(float xh, float xl, float c, float& yh
     yl = u - (yh - d);
 }
 
-// y scaled by sc, split at the grid 2^-22 (|y sc| < 1).
+// y scaled by sc, split at the grid 2^-22 (|y sc| < 1); x2 is twice the rest.
 __device__ __forceinline__ void grid_split(float yh, float yl, float sc, float& x1, float& x2) {
     x1 = __fadd_rn(__fmaf_rn(yh, sc, 3.f), -3.f);
-    x2 = __fmaf_rn(yl, sc, __fmaf_rn(yh, sc, -x1));
+    x2 = 2.f * __fmaf_rn(yl, sc, __fmaf_rn(yh, sc, -x1));
 }
 
 // Double total of a block (thread 0).
@@ -248,7 +267,7 @@ __device__ __forceinline__ double pot_block_sum(double v) {
 }
 
 // Block (I, c): targets of tile I against sources [128 I + c chunk, + chunk),
-// pairs i < j.  FP32-pipe bound: 52 operations per pair, two sources per
+// pairs i < j.  FP32-pipe bound: 54 operations per pair, two sources per
 // packed instruction.  partial[c gridDim.x + I] (0 past the end).
 template <bool SPLIT>
 __global__ void __launch_bounds__(kPotThreads, 5) potential_df_kernel(long long n, const float4* __restrict__ pos,
@@ -328,8 +347,9 @@ __global__ void __launch_bounds__(kPotThreads, 5) potential_df_kernel(long long 
                 // rounded up, so that every pair inside the kernel is caught
                 const float k2 = spline_h > 0.0 ? (float)(4.00001 * (spline_h * scd) * (spline_h * scd)) : 0.f;
                 sm.sc[w] = sc;
-                sm.e2h[w] = (float)e2;
-                sm.e2l[w] = (float)(e2 - (double)(float)e2);
+                const float e2h = (float)__dadd_rn(__dadd_rn(e2, 384.0), -384.0);  // on the grid 2^-44
+                sm.e2h[w] = e2h;
+                sm.e2l[w] = (float)(e2 - (double)e2h);
                 sm.kernel2[w] = k2;
                 sm.near2[w] = fmaxf(kPotNear2, k2);
             }
@@ -366,11 +386,11 @@ __global__ void __launch_bounds__(kPotThreads, 5) potential_df_kernel(long long 
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
                     const long long j0 = jf + k4 + 2 * half;
-                    float2 s[3], l[3], m = half ? make_float2(qm.z, qm.w) : make_float2(qm.x, qm.y);
+                    float2 s[3], l2[3], m = half ? make_float2(qm.z, qm.w) : make_float2(qm.x, qm.y);
 #pragma unroll
                     for (int x = 0; x < 3; ++x) {
                         s[x] = vadd(half ? make_float2(q1[x].z, q1[x].w) : make_float2(q1[x].x, q1[x].y), n1[x]);
-                        l[x] = vadd(half ? make_float2(q2[x].z, q2[x].w) : make_float2(q2[x].x, q2[x].y), n2[x]);
+                        l2[x] = vadd(half ? make_float2(q2[x].z, q2[x].w) : make_float2(q2[x].x, q2[x].y), n2[x]);
                     }
                     if (diag) {
                         if (j0 <= i) m.x = 0.f;
@@ -378,7 +398,7 @@ __global__ void __launch_bounds__(kPotThreads, 5) potential_df_kernel(long long 
                     }
                     const float2 B = lead_r2(s, e2h);
                     float2 y0, ny0, corr;
-                    inv_dist(s, l, e2h, e2l, B, y0, ny0, corr);
+                    inv_dist(s, l2, e2h, e2l, B, y0, ny0, corr);
                     if (!(fminf(B.x, B.y) >= near2)) {
 #pragma unroll
                         for (int u = 0; u < 2; ++u) {

@@ -53,3 +53,24 @@ def test_extent_near_the_end_of_fp32(pkg, ic, length, spline):
     """Squares of the distances are past FP32's range, at 1.5e37 some differences too."""
     x, y, z = (a * length for a in plummer(ic, 5000))
     check(pkg, x, y, z, np.full(5000, 1.0 / 5000), 0.01 * length, spline)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("eps", [0.002, 0.01, 0.05])
+def test_errors_do_not_lean(pkg, ic, eps, precision):
+    """Roundings that lean one way add up over the pairs.  The errors of FP64 sums
+    at this size are 2e-16 to 4e-16 and independent (CPU emulation, 4,096 to
+    16,384 bodies), so the mean of six has a deviation of 1.6e-16 at most; the bar
+    is three of these."""
+    errors = []
+    for seed in range(6):
+        x, y, z, _, _, _, m = ic.galaxy(5400, 600, seed=seed) if seed % 2 else ic.plummer(6000, seed=seed)
+        x, y, z = (np.float64(a) + 1e-9 for a in (x, y, z))
+        with pkg.NBodySystem(pkg.StepParams(G=1.0, eps=eps, theta=0.6), leaf_capacity=16, precision=precision) as sim:
+            sim.set_particles(x, y, z, None, None, None, m)
+            sim.prime()
+            got = sim.diagnostics(exact_potential=1)["potential"]
+            st = sim.state()
+        want = pair_sum(*st[:3], np.asarray(m, np.float32).astype(np.float64), eps, False)
+        errors.append((got - want) / abs(want))
+    assert abs(np.mean(errors)) <= 5e-16, errors
