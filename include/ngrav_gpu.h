@@ -237,9 +237,12 @@ int ngrav_gpu_get_state(ngrav_gpu_ctx* ctx, double* x, double* y, double* z, dou
 int ngrav_gpu_get_accel(ngrav_gpu_ctx* ctx, double* ax, double* ay, double* az);
 
 /* FP64 conservation diagnostics of the current state.  exact_potential:
- * 1 = exact O(N^2) pairwise potential on the GPU, every pair term to FP64
- *     accuracy (in FP64 below 4,096 particles, as a pair of floats above,
- *     with FP64 sums; the sum's error is that of FP64 terms);
+ * 1 = exact O(N^2) pairwise potential on the GPU, to the accuracy of an FP64
+ *     sum (a few 1e-16 of it).  Below 4,096 particles and with masses of both
+ *     signs every pair term is FP64; else a term is a pair of floats, good to
+ *     2^-42 to 2^-46 of itself (rms; 2^-38.8 at worst) with errors that average
+ *     out, and FP64 where 32 sources of a particle hold more than 2^-12 of the
+ *     energy.  Sums are FP64;
  * 2 = the same pair set with FP32 pair terms and FP64 sums (the offset of a
  *     pair formed from the double-float positions, so its error is of order
  *     2^-24 of the separation; Plummer softening, a spline run takes mode 1),

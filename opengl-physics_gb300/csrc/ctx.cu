@@ -926,12 +926,12 @@ int ngrav_gpu_diagnostics(ngrav_gpu_ctx* ctx, int exact_potential, ngrav_gpu_dia
     double com[3] = {s1[1], s1[2], s1[3]};
     if (M > 0.0)
         for (double& c : com) c /= M;
-    launch_diag_pass2(n, ctx->P, split, com[0], com[1], com[2], ctx->dpartial, ctx->stream);
-    NG_CUDA(cudaMemcpyAsync(h.data(), ctx->dpartial, sizeof(double) * 3 * nb, cudaMemcpyDeviceToHost, ctx->stream));
+    launch_diag_pass2(n, ctx->P, split, com[0], com[1], com[2], M, ctx->dpartial, ctx->stream);
+    NG_CUDA(cudaMemcpyAsync(h.data(), ctx->dpartial, sizeof(double) * 5 * nb, cudaMemcpyDeviceToHost, ctx->stream));
     NG_CUDA(cudaStreamSynchronize(ctx->stream));
-    double L[3] = {0, 0, 0};
+    double L[5] = {0, 0, 0, 0, 0};
     for (int b = 0; b < nb; ++b)
-        for (int k = 0; k < 3; ++k) L[k] += h[3 * b + k];
+        for (int k = 0; k < 5; ++k) L[k] += h[5 * b + k];
     out->kinetic = s1[4];
     for (int k = 0; k < 3; ++k) {
         out->com[k] = com[k];
@@ -956,7 +956,9 @@ int ngrav_gpu_diagnostics(ngrav_gpu_ctx* ctx, int exact_potential, ngrav_gpu_dia
         for (int b = 0; b < pb; ++b) pot += hp[b];
         out->potential = ctx->opts.G * pot;
     } else if (exact) {
-        launch_potential(n, ctx->P, split, ctx->opts.eps * ctx->opts.eps, spline_h(ctx), ctx->dpartial, ctx->stream);
+        const double eps2 = ctx->opts.eps * ctx->opts.eps;
+        launch_potential(n, ctx->P, split, eps2, spline_h(ctx), potential_large(M, 0.5 * L[3], L[4], eps2),
+                         ctx->dpartial, ctx->stream);
         NG_CUDA(cudaMemcpyAsync(h.data(), ctx->dpartial, sizeof(double) * npb, cudaMemcpyDeviceToHost,
                                 ctx->stream));
         NG_CUDA(cudaStreamSynchronize(ctx->stream));

@@ -20,16 +20,18 @@ void launch_download(long long n, const int* id, const float4* a, const float4* 
 void launch_inverse_id(long long n, const int* id, int* inv, cudaStream_t s);
 int diag_blocks(long long n);
 void launch_diag_pass1(long long n, const Particles& P, bool split, double* partial, cudaStream_t s);
-void launch_diag_pass2(long long n, const Particles& P, bool split, double cx, double cy, double cz, double* partial,
-                       cudaStream_t s);
-// potential.cu: the exact pair potential, one partial sum per block.
+void launch_diag_pass2(long long n, const Particles& P, bool split, double cx, double cy, double cz, double mass,
+                       double* partial, cudaStream_t s);
+// potential.cu: the exact pair potential, one partial sum per block.  `large`
+// (potential_large): sums above it are FP64 throughout.
 int potential_blocks(long long n);
+double potential_large(double mass, double pairs, double inertia, double eps2);
 // Exact pair potential with FP32 pair terms and FP64 sums (Plummer).
 int potential_f32_blocks(long long n, int sm_count);
 void launch_potential_f32(long long n, const Particles& P, bool split, double eps2, int blocks, double* partial,
                           cudaStream_t s);
-void launch_potential(long long n, const Particles& P, bool split, double eps2, double spline_h, double* partial,
-                      cudaStream_t s);
+void launch_potential(long long n, const Particles& P, bool split, double eps2, double spline_h, double large,
+                      double* partial, cudaStream_t s);
 int sampler_shares(long long n, int nslots, int sm_count);
 // FP64 pairs (one block per target), or FP32 pairs tiled over `shares`
 // source shares with FP64 totals (partial: shares * 3 * nslots doubles).

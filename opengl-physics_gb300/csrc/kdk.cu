@@ -321,13 +321,18 @@ __global__ void __launch_bounds__(kDiagThreads) diag_pass1_kernel(long long n, c
     }
 }
 
-// Pass 2: per block {Lx, Ly, Lz} about the given COM.
+// Pass 2: per block {Lx, Ly, Lz} about the given COM, and the sums of m_i m_j
+// over pairs (twice) and of m r^2, which tell the pair potential how large its
+// terms can be (potential_large).  A particle's partners weigh M - m, a difference
+// that is exact where one particle holds nearly all of M.  The sum is -infinity if
+// a mass is negative.
 __global__ void __launch_bounds__(kDiagThreads) diag_pass2_kernel(long long n, const float4* __restrict__ pos,
                                                                   const float4* __restrict__ plo,
                                                                   const float4* __restrict__ vel,
                                                                   const float4* __restrict__ vlo, double cx,
-                                                                  double cy, double cz, double* __restrict__ partial) {
-    double L[3] = {0, 0, 0};
+                                                                  double cy, double cz, double mass,
+                                                                  double* __restrict__ partial) {
+    double L[5] = {0, 0, 0, 0, 0};
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         double x, y, z, vx, vy, vz, m;
         load_state_d(i, pos, plo, vel, vlo, x, y, z, vx, vy, vz, m);
@@ -335,11 +340,13 @@ __global__ void __launch_bounds__(kDiagThreads) diag_pass2_kernel(long long n, c
         L[0] += m * (ry * vz - vy * rz);
         L[1] += m * (rz * vx - vz * rx);
         L[2] += m * (rx * vy - vx * ry);
+        L[3] += m < 0.0 ? -1.0 / 0.0 : m * (mass - m);
+        L[4] += m * (rx * rx + ry * ry + rz * rz);
     }
     __shared__ double sh[32];
-    for (int k = 0; k < 3; ++k) {
+    for (int k = 0; k < 5; ++k) {
         const double t = block_sum_d(L[k], sh);
-        if (threadIdx.x == 0) partial[blockIdx.x * 3 + k] = t;
+        if (threadIdx.x == 0) partial[blockIdx.x * 5 + k] = t;
     }
 }
 
@@ -350,10 +357,10 @@ void launch_diag_pass1(long long n, const Particles& P, bool split, double* part
                                                                split ? P.vlo : nullptr, partial);
 }
 
-void launch_diag_pass2(long long n, const Particles& P, bool split, double cx, double cy, double cz, double* partial,
-                       cudaStream_t s) {
+void launch_diag_pass2(long long n, const Particles& P, bool split, double cx, double cy, double cz, double mass,
+                       double* partial, cudaStream_t s) {
     diag_pass2_kernel<<<diag_blocks(n), kDiagThreads, 0, s>>>(n, P.pos, split ? P.plo : nullptr, P.vel,
-                                                               split ? P.vlo : nullptr, cx, cy, cz,
+                                                               split ? P.vlo : nullptr, cx, cy, cz, mass,
                                                               partial);
 }
 

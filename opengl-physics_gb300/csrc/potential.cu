@@ -30,8 +30,10 @@
 //  * a pair nearer than E/16 is formed again from the particles' own double-float
 //    positions with error-free differences (refine_pair), and pairs inside the
 //    spline's kernel or at r = 0 take the FP64 formula;
-//  * 32 sources whose numbers FP32 does not hold are summed in FP64 (frame_f64),
-//    and so are all pairs below kPotDfMin.
+//  * where a target's 32 sources hold more than 2^-12 of the energy
+//    (potential_large), or FP32 does not hold their numbers, they are summed in
+//    FP64 (frame_f64);
+//  * with masses of both signs, and below kPotDfMin, all pairs are FP64.
 // Emulated on the CPU with exact rounding against 80-bit sums (Plummer spheres in
 // double-float and in FP32 positions, eps 0 to 0.05), the sum's relative error, rms
 // and worst, and that of FP64 terms: n = 1,000 6e-16, 1e-15 and 2e-16, 4e-16; 2,048
@@ -51,6 +53,7 @@
 #include "softening.cuh"
 
 #include <algorithm>
+#include <cmath>
 
 namespace ngrav {
 
@@ -172,7 +175,7 @@ __device__ __forceinline__ double pair_phi(double dx, double dy, double dz, doub
 }
 
 // The sources [jf, j_end) after target i, in FP64: of a frame whose numbers FP32
-// does not hold.
+// does not hold, or whose sum is a large part of the energy.
 __device__ __noinline__ double frame_f64(const float4* __restrict__ pos, const float4* __restrict__ plo, float4 th,
                                          float4 tl, long long i, long long jf, long long j_end, double eps2,
                                          double spline_h) {
@@ -272,7 +275,7 @@ __device__ __forceinline__ double pot_block_sum(double v) {
 template <bool SPLIT>
 __global__ void __launch_bounds__(kPotThreads, 5) potential_df_kernel(long long n, const float4* __restrict__ pos,
                                                                       const float4* __restrict__ plo, double eps2,
-                                                                      double spline_h, long long chunk,
+                                                                      double spline_h, double large, long long chunk,
                                                                       double* __restrict__ partial) {
     __shared__ PotStage sm;
     __shared__ unsigned s_rho;
@@ -373,6 +376,7 @@ __global__ void __launch_bounds__(kPotThreads, 5) potential_df_kernel(long long 
                 n1[k] = splat<float2>(-x1);
                 n2[k] = splat<float2>(-x2);
             }
+            const double before = acc;
             const bool diag = jf < i0 + kPotThreads;  // sources at or before some target
             float2 A = make_float2(0.f, 0.f), R = A;
             for (int k4 = 0; k4 < kPotSub; k4 += 4) {
@@ -434,8 +438,11 @@ __global__ void __launch_bounds__(kPotThreads, 5) potential_df_kernel(long long 
             }
             float S, er;
             sum2(A.x, A.y, S, er);
-            acc = fma((double)S, unit, acc);
-            acc = fma((double)(er + (R.x + R.y)), unit, acc);
+            const double high = (double)S * unit;
+            if (high * (double)th.w > large)
+                acc = before + frame_f64(pos, SPLIT ? plo : nullptr, th, tl, i, jf, min(jf + kPotSub, j_end), eps2, spline_h);
+            else
+                acc = fma((double)(er + (R.x + R.y)), unit, acc + high);
         }
     }
     const double t = pot_block_sum(have ? -(double)th.w * acc : 0.0);
@@ -487,17 +494,33 @@ __global__ void __launch_bounds__(kPotThreads) potential_f64_kernel(long long n,
     if (tid == 0) *out = t;
 }
 
-void launch_potential(long long n, const Particles& P, bool split, double eps2, double spline_h, double* partial,
-                      cudaStream_t s) {
+// A target's sum over 32 sources above this is formed in FP64: 2^-12 of a lower
+// bound of the energy, so that what is left are at least 2^12 sums of independent
+// errors, the worst of 2^-42 each (rms), and their mean is good to 2^-48.  Sums that
+// large are few: the bound is about half of the energy of a Plummer sphere or a
+// galaxy, and 32 sources hold 2^-18 of it on average at n = 4,096.  The bound:
+// 1/sqrt(r^2 + eps^2) is convex in r^2, so its mean over pairs is at least its
+// value at their mean r^2, which `inertia`, the sum of m r^2 about the centre of
+// mass, gives times the mass; the spline's potential is nowhere weaker than
+// 1/sqrt(r^2 + h^2).  With masses of both signs (pairs < 0, diag_pass2_kernel) no
+// bound holds: NaN, and every pair is FP64.
+double potential_large(double mass, double pairs, double inertia, double eps2) {
+    if (!(pairs >= 0.0)) return std::nan("");
+    return pairs > 0.0 ? pairs / std::sqrt(mass * inertia / pairs + eps2) / 4096.0 : 0.0;
+}
+
+void launch_potential(long long n, const Particles& P, bool split, double eps2, double spline_h, double large,
+                      double* partial, cudaStream_t s) {
     const dim3 grid((unsigned)pot_tiles(n), (unsigned)pot_chunks(n));
     const long long chunk = potential_chunk(n);
-    if (n < kPotDfMin)
+    if (n < kPotDfMin || !(large >= 0.0))
         potential_f64_kernel<<<grid, kPotThreads, 0, s>>>(n, P.pos, split ? P.plo : nullptr, eps2, spline_h, chunk,
                                                           partial);
     else if (split)
-        potential_df_kernel<true><<<grid, kPotThreads, 0, s>>>(n, P.pos, P.plo, eps2, spline_h, chunk, partial);
+        potential_df_kernel<true><<<grid, kPotThreads, 0, s>>>(n, P.pos, P.plo, eps2, spline_h, large, chunk, partial);
     else
-        potential_df_kernel<false><<<grid, kPotThreads, 0, s>>>(n, P.pos, nullptr, eps2, spline_h, chunk, partial);
+        potential_df_kernel<false><<<grid, kPotThreads, 0, s>>>(n, P.pos, nullptr, eps2, spline_h, large, chunk,
+                                                                partial);
 }
 
 }  // namespace ngrav

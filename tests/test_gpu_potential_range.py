@@ -55,6 +55,44 @@ def test_extent_near_the_end_of_fp32(pkg, ic, length, spline):
     check(pkg, x, y, z, np.full(5000, 1.0 / 5000), 0.01 * length, spline)
 
 
+def heavy_pair(ic, n, gap):
+    """A wide set with bodies 1 and 20 `gap` of its extent apart."""
+    x, y, z = plummer(ic, n)
+    d = gap / 3 * max(np.abs(a).max() for a in (x, y, z))
+    x[20], y[20], z[20] = x[1] + d, y[1] - 2 * d, z[1] + 2 * d * (1 + 1e-11)
+    return x, y, z
+
+
+@pytest.mark.parametrize("sort", [False, True])
+@pytest.mark.parametrize("n", [4096, 5000, 9000])
+@pytest.mark.parametrize("gap", [0.0442, 0.06, 0.1, 0.3])
+def test_heavy_pair_in_a_wide_frame(pkg, ic, gap, n, sort):
+    """Two bodies that carry nearly all of the energy, from just above the 1/16 of
+    their frame's extent below which a pair is formed by itself."""
+    m = np.full(n, 1e-9 / n)
+    m[1], m[20] = 0.7, 0.3
+    check(pkg, *heavy_pair(ic, n, gap), m, 0.0, sort=sort)
+
+
+@pytest.mark.parametrize("gap", [0.0442, 0.06, 0.1, 0.3])
+def test_masses_of_both_signs(pkg, ic, gap):
+    """The same with a negative mass: what a pair's share is of the sum of sizes
+    says nothing about its share of the sum."""
+    m = np.random.default_rng(9).uniform(-1.0, 1.0, 5000) * 1e-9 / 5000
+    m[1], m[20] = 0.7, -0.3
+    check(pkg, *heavy_pair(ic, 5000, gap), m, 0.0)
+
+
+@pytest.mark.parametrize("heavy", [3, 200])
+def test_few_heavy_bodies(pkg, ic, heavy):
+    """A handful of bodies, and a few hundred, with all but 1e-6 of the mass."""
+    x, y, z = plummer(ic, 6000)
+    rng = np.random.default_rng(heavy)
+    m = rng.uniform(0.5, 1.5, 6000) * 1e-6 / 6000
+    m[rng.choice(6000, heavy, replace=False)] = rng.uniform(0.5, 1.5, heavy) / heavy
+    check(pkg, x, y, z, m, 1e-3, sort=True)
+
+
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("eps", [0.002, 0.01, 0.05])
 def test_errors_do_not_lean(pkg, ic, eps, precision):
