@@ -598,7 +598,12 @@ int ngrav_gpu_create(ngrav_gpu_ctx** out, const ngrav_gpu_opts* opts) {
         NG_CUDA(cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, ctx->opts.device));
         NG_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
         NG_CUDA(cudaMalloc((void**)&ctx->C, sizeof(Counters)));
+        // dynamic shared-memory limits: they belong to a device, so every context
+        // sets them on its own
+        sort_set_attributes();
         lmac_set_attributes();
+        lmac_data_set_attributes();
+        lmac_train_set_attributes();
         walk_pp_set_attributes();
         NG_CUDA(cudaGetLastError());
         // Walk: up to 32 resident warps per SM (latency-bound traversal);

@@ -38,7 +38,10 @@ int sampler_shares(long long n, int nslots, int sm_count);
 void launch_sampler(long long n, const Particles& P, bool split, const int* slots, int nslots, double eps2,
                     double spline_h, bool fp64_pairs, double* out, double* partial, int shares, cudaStream_t s);
 void launch_reset_counters(Counters* C, cudaStream_t s);
+void sort_set_attributes();
 void lmac_set_attributes();
+void lmac_data_set_attributes();
+void lmac_train_set_attributes();
 int walk_warps_per_block();
 int walk_blocks_per_sm();
 int eval_warps_per_block();

@@ -655,11 +655,21 @@ constexpr int kRsSingleMax = 1024 * kRsItems;
 // tiles) takes 78 us with three and 63 with two, of 131,071 (32 tiles) 82 and 97.
 constexpr int kRsFewTiles = 12;
 
+constexpr int rs_single_smem(int threads) {
+    return threads * kRsItems * (int)(sizeof(unsigned long long) + sizeof(unsigned));
+}
+
 template <int THREADS>
 static void launch_single(SortBuffers& sb, int n, int passes, int shift0, cudaStream_t s) {
-    const int smem = THREADS * kRsItems * (int)(sizeof(unsigned long long) + sizeof(unsigned));
-    cudaFuncSetAttribute(rs_single_kernel<THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    rs_single_kernel<THREADS><<<1, THREADS, smem, s>>>(sb.keys, sb.vals, n, passes, shift0);
+    rs_single_kernel<THREADS><<<1, THREADS, rs_single_smem(THREADS), s>>>(sb.keys, sb.vals, n, passes, shift0);
+}
+
+void sort_set_attributes() {
+    const auto kind = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaFuncSetAttribute(rs_single_kernel<kRsThreads>, kind, rs_single_smem(kRsThreads));
+    cudaFuncSetAttribute(rs_single_kernel<1024>, kind, rs_single_smem(1024));
+    cudaFuncSetAttribute(rs_scatter_kernel<false>, kind, (int)kRsScatterSmem);
+    cudaFuncSetAttribute(rs_scatter_kernel<true>, kind, (int)kRsScatterSmem);
 }
 
 long long radix_hist_size(long long n) { return ((n + kRsTile - 1) / kRsTile + 1) * kRsBins; }
@@ -677,14 +687,6 @@ int radix_sort_pairs(SortBuffers& sb, long long n, int passes, int shift0, cudaS
         return 1;
     }
     const int nb = (int)((n + kRsTile - 1) / kRsTile);
-    static bool attr_done = false;
-    if (!attr_done) {
-        cudaFuncSetAttribute(rs_scatter_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kRsScatterSmem);
-        cudaFuncSetAttribute(rs_scatter_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kRsScatterSmem);
-        attr_done = true;
-    }
     const bool few = nb <= kRsFewTiles;
     unsigned* totals = sb.hist + (long long)nb * kRsBins;
     unsigned long long *kin = sb.keys, *kout = sb.keys_alt;

@@ -239,15 +239,15 @@ __global__ void lmac_feature_kernel(NodeArrays T, const int2* __restrict__ pairs
     }
 }
 
+constexpr int kRecSmem = (int)sizeof(int) * kRecWarps * kRecStack;
+
+void lmac_data_set_attributes() {
+    cudaFuncSetAttribute(lmac_record_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRecSmem);
+}
+
 void launch_lmac_record(const NodeArrays& T, const Counters* C, const int* leaf_list, const LmacRecordParams& rp,
                         int blocks, cudaStream_t s) {
-    const size_t smem = sizeof(int) * kRecWarps * kRecStack;
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(lmac_record_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr = true;
-    }
-    lmac_record_kernel<<<blocks, kRecWarps * 32, smem, s>>>(T, C, leaf_list, rp);
+    lmac_record_kernel<<<blocks, kRecWarps * 32, kRecSmem, s>>>(T, C, leaf_list, rp);
 }
 
 void launch_lmac_amin(const NodeArrays& T, const Counters* C, const int* leaf_list, const float4* acc,

@@ -204,14 +204,13 @@ void launch_lmac_make_batch(const float* X, const float* r, long long n, const L
     lmac_make_batch_kernel<<<b, 256, 0, s>>>(X, r, n, norm, nb, seed, u_range, standardise ? 1 : 0, Xb, yb, wb);
 }
 
+void lmac_train_set_attributes() {
+    cudaFuncSetAttribute(lmac_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lmac_grad_smem_bytes());
+}
+
 void launch_lmac_grad(const float* Xb, const float* yb, const float* wb, int nb, const float* P, float scale,
                       float* partial, float* stats, cudaStream_t s) {
-    static bool attr = false;
     const size_t smem = lmac_grad_smem_bytes();
-    if (!attr) {
-        cudaFuncSetAttribute(lmac_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr = true;
-    }
     lmac_grad_kernel<<<lmac_grad_blocks(nb), kTrainThreads, smem, s>>>(Xb, yb, wb, nb, P, scale, partial, stats);
 }
 

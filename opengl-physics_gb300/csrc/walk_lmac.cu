@@ -482,8 +482,8 @@ __global__ void __launch_bounds__(kLwThreads) lmac_tc_forward_kernel(const LmacD
 
 static size_t tc_smem_bytes() { return sizeof(LmacTiles) + 1024; }
 
-// Dynamic shared-memory limits of the tensor-core kernels, set once at
-// context creation (never inside a graph capture).
+// Dynamic shared-memory limits of the tensor-core kernels, set at context
+// creation (never inside a graph capture).
 void lmac_set_attributes() {
     const int smem = (int)tc_smem_bytes();
     cudaFuncSetAttribute(lmac_infer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

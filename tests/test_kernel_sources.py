@@ -28,3 +28,23 @@ def test_aligned_instructions_follow_a_reconvergence(name):
             assert before.endswith("__syncwarp()") or ".aligned" in before, s
         before = s
     assert found
+
+
+def test_attributes_are_set_for_every_context():
+    """A kernel's attributes belong to a device: set once per process, behind a
+    static flag, they are missing on the next device that a context is made on.
+    They are set at context creation only, and no launcher keeps a flag."""
+    setters = set()
+    for name in sorted(os.listdir(CSRC)):
+        function = ""
+        with open(os.path.join(CSRC, name)) as f:
+            for line in f:
+                assert "static bool" not in line, (name, line)
+                start = re.match(r"[a-z][\w:<>*& ]* \**(\w+)\(", line)
+                function = start.group(1) if start else function
+                if "cudaFuncSetAttribute(" in line:
+                    assert function.endswith("_set_attributes"), (name, function)
+                    setters.add(function)
+    with open(os.path.join(CSRC, "ctx.cu")) as f:
+        create = f.read().split("int ngrav_gpu_create(")[1].split("\nvoid ngrav_gpu_destroy")[0]
+    assert setters and all(fn + "();" in create for fn in setters), setters
