@@ -232,15 +232,18 @@ struct Forest {
     float4* frame = nullptr;          // per system: its key frame (kFrame)
 };
 
+// Error-free steps.  Every rounding is asked for by name: an operand may be a
+// product after inlining, and one fused into the sum, but not into its error,
+// would be counted twice.
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
-    s = a + b;
-    const float bb = s - a;
-    e = (a - (s - bb)) + (b - bb);
+    s = __fadd_rn(a, b);
+    const float bb = __fsub_rn(s, a);
+    e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
 }
 
 __device__ __forceinline__ void fast_two_sum(float a, float b, float& s, float& e) {
-    s = a + b;
-    e = b - (s - a);
+    s = __fadd_rn(a, b);
+    e = __fsub_rn(b, __fsub_rn(s, a));
 }
 
 // Offset of a double-float coordinate (h + l) from a double-float centre
@@ -248,18 +251,16 @@ __device__ __forceinline__ void fast_two_sum(float a, float b, float& s, float& 
 __device__ __forceinline__ void df_offset(float h, float l, float ch, float cl, float& oh, float& ol) {
     float s, e;
     two_sum(h, -ch, s, e);
-    fast_two_sum(s, e + (l - cl), oh, ol);
+    fast_two_sum(s, __fadd_rn(e, __fsub_rn(l, cl)), oh, ol);
 }
 
-// (h, l) += d for a double-float pair: error-free two-sum, renormalised.
-__device__ __forceinline__ void df_add(float& h, float& l, float d) {
-    const float s = h + d;
-    const float bb = s - h;
-    const float e = (h - (s - bb)) + (d - bb);
-    const float l2 = l + e;
-    const float h2 = s + l2;
-    l = l2 - (h2 - s);
-    h = h2;
+// (h, l) += m (oh + ol) for a double-float pair, the product of the high parts exact.
+__device__ __forceinline__ void df_add_prod(float& h, float& l, float m, float oh, float ol) {
+    const float p = __fmul_rn(m, oh);
+    const float pe = __fmaf_rn(m, ol, __fmaf_rn(m, oh, -p));
+    float t, e;
+    two_sum(h, p, t, e);
+    fast_two_sum(t, __fadd_rn(l, __fadd_rn(e, pe)), h, l);
 }
 
 // Bounding box of double-float coordinates, compared as pairs: the high part is
@@ -348,9 +349,9 @@ __device__ __forceinline__ void box_publish(DfBox& b, bool bad, Counters* C) {
 // pair when vl is given (split precision), else in FP32.
 __device__ __forceinline__ void kick_v(float4& v, float4* vl, float h, const float4& a) {
     if (vl) {
-        df_add(v.x, vl->x, h * a.x);
-        df_add(v.y, vl->y, h * a.y);
-        df_add(v.z, vl->z, h * a.z);
+        df_add_prod(v.x, vl->x, h, a.x, 0.f);
+        df_add_prod(v.y, vl->y, h, a.y, 0.f);
+        df_add_prod(v.z, vl->z, h, a.z, 0.f);
     } else {
         v.x = fmaf(h, a.x, v.x);
         v.y = fmaf(h, a.y, v.y);

@@ -323,7 +323,7 @@ __device__ __forceinline__ void finish_row(const Total& g, int h, int row, int f
         if (SPLIT) {
             float* l = reinterpret_cast<float*>(vlo + slot) + axis;
             float vh = *v, vl = *l;
-            df_add(vh, vl, wp.hdt * a);
+            df_add_prod(vh, vl, wp.hdt, a, 0.f);
             *v = vh;
             *l = vl;
         } else {

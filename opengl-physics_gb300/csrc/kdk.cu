@@ -221,13 +221,9 @@ __global__ void __launch_bounds__(256) kick_drift_kernel(long long n, float4* __
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 // two-sum of hi + d, error folded into lo, then renormalised
-                const float s = ph[k] + dv[k];
-                const float bb = s - ph[k];
-                const float e = (ph[k] - (s - bb)) + (dv[k] - bb);
-                const float lo2 = pl[k] + e;
-                const float h2 = s + lo2;
-                pl[k] = lo2 - (h2 - s);
-                ph[k] = h2;
+                float s, e;
+                two_sum(ph[k], dv[k], s, e);
+                fast_two_sum(s, __fadd_rn(pl[k], e), ph[k], pl[k]);
             }
             plo[i] = l;
         } else {
@@ -506,13 +502,9 @@ __global__ void __launch_bounds__(256) block_kick_drift_kernel(long long n, floa
                                  fmaf(dtmin, v.z, dtmin * vl.z)};
 #pragma unroll
             for (int k = 0; k < 3; ++k) {  // (hi, lo) += d with an error-free two-sum
-                const float s = ph[k] + dv[k];
-                const float bb = s - ph[k];
-                const float err = (ph[k] - (s - bb)) + (dv[k] - bb);
-                const float lo = pl[k] + err;
-                const float hi2 = s + lo;
-                pl[k] = lo - (hi2 - s);
-                ph[k] = hi2;
+                float s, e;
+                two_sum(ph[k], dv[k], s, e);
+                fast_two_sum(s, __fadd_rn(pl[k], e), ph[k], pl[k]);
             }
             plo[i] = l;
         } else {

@@ -384,20 +384,12 @@ __device__ __forceinline__ void write_walk_record(NodeArrays& T, int node, doubl
 // of a leaf counts, one where there are many, which spares the reductions.
 // Before and now: 297 k leaves (4 Mi bodies) 278 and 156 us, 462 leaves (2,048
 // bodies) 27 and 13 us; eight lanes throughout took 185 us at 297 k leaves.
-// (Sh, Sl) += m * (oh + ol), the product of the high parts exact.
-__device__ __forceinline__ void df_add_prod(float& Sh, float& Sl, float m, float oh, float ol) {
-    const float p = m * oh;
-    const float pe = fmaf(m, oh, -p) + m * ol;
-    float t, e;
-    two_sum(Sh, p, t, e);
-    fast_two_sum(t, Sl + (e + pe), Sh, Sl);
-}
 
 // (ah, al) += (bh, bl)
 __device__ __forceinline__ void df_add(float& ah, float& al, float bh, float bl) {
     float t, e;
     two_sum(ah, bh, t, e);
-    fast_two_sum(t, al + (bl + e), ah, al);
+    fast_two_sum(t, __fadd_rn(al, __fadd_rn(bl, e)), ah, al);
 }
 
 __device__ __forceinline__ void df_add_xor(float& h, float& l, int o) {

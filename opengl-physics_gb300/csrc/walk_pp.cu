@@ -88,13 +88,6 @@ __device__ __forceinline__ float2 pp_mul(float2 a, float2 b) { return __fmul2_rn
 __device__ __forceinline__ float2 pp_fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 pp_dup(float v) { return make_float2(v, v); }
 
-// a + b = s + e exactly, whichever is larger.
-__device__ __forceinline__ void pp_sum2(float a, float b, float& s, float& e) {
-    const float t = a + b, bb = t - a;
-    e = (a - (t - bb)) + (b - bb);
-    s = t;
-}
-
 // Two sources or node centres (double-float) of one lane, and their members.
 struct PpPair {
     float2 x, y, z, m;
@@ -123,8 +116,9 @@ struct PpSum {
     __device__ __forceinline__ void add(const float v[3]) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            float e;
-            pp_sum2(s[k], v[k], s[k], e);
+            float t, e;
+            two_sum(s[k], v[k], t, e);
+            s[k] = t;
             low[k] += e;
         }
     }

@@ -48,3 +48,16 @@ def test_attributes_are_set_for_every_context():
     with open(os.path.join(CSRC, "ctx.cu")) as f:
         create = f.read().split("int ngrav_gpu_create(")[1].split("\nvoid ngrav_gpu_destroy")[0]
     assert setters and all(fn + "();" in create for fn in setters), setters
+
+
+@pytest.mark.parametrize("name,functions", [("engine.cuh", ["two_sum", "fast_two_sum", "df_offset", "df_add_prod"]),
+                                            ("tree.cu", ["df_add"])])
+def test_error_free_steps_name_their_roundings(name, functions):
+    """A plain float sum may be fused with the product that an operand comes from,
+    by the compiler's choice, and an error-free step is none any more."""
+    with open(os.path.join(CSRC, name)) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    for fn in functions:
+        bodies = re.findall(r"__forceinline__ void " + fn + r"\([^)]*\) \{(.*?)\n\}", text, re.S)
+        assert len(bodies) == 1, fn
+        assert not re.search(r" [-+*] ", bodies[0]), bodies[0]
