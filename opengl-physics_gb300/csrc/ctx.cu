@@ -251,7 +251,7 @@ void enqueue_eval(ngrav_gpu_ctx* ctx, bool bbox_ready, bool kick, float hdt) {
         // kernel; block timesteps take the geometric test on their targets
         // (ComputeAccelBarnesHutTargets, Solvers.cpp:384-405)
         rec(ctx, 5);
-        launch_walk_pp(ctx->T, ctx->C, P, ctx->TB.leaf_list, wp, ctx->block_on ? 0 : 1, ctx->alpha, nullptr,
+        launch_walk_pp(ctx->T, ctx->C, P, ctx->TB.leaf_list, wp, ctx->block_on ? 0 : 1, ctx->alpha,
                        ctx->block_on ? ctx->block_args : nullptr, ctx->block_base, n, ctx->TB.leaf_before,
                        ctx->TB.leaf_start, ctx->LB.nwarps, s);
         rec(ctx, 6);

@@ -57,14 +57,14 @@ void launch_forest_diag(const Particles& P, bool split, const Forest& F, double*
 void launch_forest_potential(const Particles& P, bool split, const Forest& F, double eps2, int chunks, double* part,
                              cudaStream_t s);
 
-// walk_pp.cu: the per-particle walk (relative MAC, target subsets), with the
+// walk_pp.cu: the per-particle walk (relative MAC, block timesteps), with the
 // force sums and the closing kick.
-// block = {sub, rmax}: block-timestep mode (nullptr: every particle).
+// block = {sub, rmax}: the particles whose step ends there (nullptr: all).
 // before / starts: TreeBuffers::leaf_before and leaf_start.
 void walk_pp_set_attributes();
 void launch_walk_pp(const NodeArrays& T, Counters* C, const Particles& P, const int* leaf_list, const WalkParams& wp,
-                    int relative, double alpha, const unsigned char* targets, const int* block, double block_base,
-                    long long n, const unsigned* before, const unsigned* starts, int nwarps, cudaStream_t s);
+                    int relative, double alpha, const int* block, double block_base, long long n,
+                    const unsigned* before, const unsigned* starts, int nwarps, cudaStream_t s);
 // kdk.cu: block timesteps
 void launch_frame_download(long long n, const int* id, const float4* pos, const float4* plo, const float4* vel,
                            const float4* vlo, float* opos, float* ovel, cudaStream_t s);

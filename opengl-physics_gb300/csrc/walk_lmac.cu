@@ -119,15 +119,6 @@ __device__ __forceinline__ uint4 lmac_row(const float f[kLmacIn], const WalkPara
     return v;
 }
 
-__device__ __forceinline__ bool geometric_accept(const float4 A, const float4 Cw, const float4 D, const float4 gA,
-                                                 const float4 gD, float gR, float theta2) {
-    const float dx = (A.x - gA.x) + (D.x - gD.x);
-    const float dy = (A.y - gA.y) + (D.y - gD.y);
-    const float dz = (A.z - gA.z) + (D.z - gD.z);
-    const float worst = sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) - gR;
-    return worst > 0.f && Cw.y * Cw.y < theta2 * worst * worst;
-}
-
 template <int STACK, int MINB>
 __global__ void __launch_bounds__(kLwThreads, MINB) walk_lmac_round_kernel(NodeArrays T, Counters* C,
                                                                         const int* __restrict__ leaf_list,

@@ -60,7 +60,6 @@ struct PpParams {
     int n;                            // particles
     const unsigned* before;           // per slot: leaves that start before it
     const unsigned* starts;           // per slot: 1 if a leaf starts there
-    const unsigned char* targets;     // per slot: compute this particle (NULL: all)
     // block timesteps (System::BlockStep): only particles whose rung step
     // (rung in vel.w) ends at finest substep `sub` + 1, each closing with its
     // own half-kick 0.5 base / 2^rung
@@ -307,7 +306,6 @@ __global__ void __launch_bounds__(kPpThreads, 4) walk_pp_kernel(NodeArrays T, Co
         if (si >= nslices) break;
         const int own = si * kPpTargets, slot = own + lane;
         bool mine = lane < kPpTargets && slot < pp.n;
-        if (mine && pp.targets) mine = pp.targets[slot] != 0;
         float hdt_mine = wp.hdt;
         if (mine && pp.block) {
             const int rung = (int)P.vel[slot].w;
@@ -524,8 +522,8 @@ void walk_pp_set_attributes() {
 }
 
 void launch_walk_pp(const NodeArrays& T, Counters* C, const Particles& P, const int* leaf_list, const WalkParams& wp,
-                    int relative, double alpha, const unsigned char* targets, const int* block, double block_base,
-                    long long n, const unsigned* before, const unsigned* starts, int nwarps, cudaStream_t s) {
+                    int relative, double alpha, const int* block, double block_base, long long n,
+                    const unsigned* before, const unsigned* starts, int nwarps, cudaStream_t s) {
     PpParams pp;
     pp.n = (int)n;
     pp.before = before;
@@ -533,7 +531,6 @@ void launch_walk_pp(const NodeArrays& T, Counters* C, const Particles& P, const 
     pp.relative = relative;
     pp.alpha = (float)alpha;
     pp.alpha_d = alpha;
-    pp.targets = targets;
     pp.block = block ? 1 : 0;
     pp.sub = block ? block[0] : 0;
     pp.rmax = block ? block[1] : 0;
