@@ -114,7 +114,8 @@ typedef struct ngrav_gpu_stats {
     long long groups;      /* target groups (leaves) walked */
     int nodes, leaves, levels, max_leaf_count;
     int depth_limited_leaves; /* leaves at the 21-level key limit holding > leaf_capacity */
-    int walk_stack_max;
+    int walk_stack_max;    /* four times the opened nodes that waited on the deepest walk stack
+                            * (walk_stack / 4 of them fit in shared memory) */
     unsigned status_bits;  /* raw device status word of the last evaluation */
     long long force_evals; /* force evaluations since the context was created */
     long long n;
@@ -340,8 +341,9 @@ typedef struct ngrav_gpu_tune_report {
 
 int ngrav_gpu_default_tune_opts(ngrav_gpu_tune_opts* o);
 int ngrav_gpu_autotune(ngrav_gpu_ctx* ctx, const ngrav_gpu_tune_opts* o, ngrav_gpu_tune_report* out);
-/* Set the tuned kernel shapes directly: p2p_tile in {64, 128, 256} (0: 256),
- * walk_stack in {1024, 2048, 4096}. */
+/* Set the tuned kernel shapes directly: p2p_tile, the sources per near batch of
+ * the evaluation, at most 64 or 128, or 256 for as many as there is room for (up
+ * to 1,024; 0: the same); walk_stack in {1024, 2048, 4096}. */
 int ngrav_gpu_set_tuning(ngrav_gpu_ctx* ctx, int p2p_tile, int walk_stack);
 
 /* ---- ensembles of independent systems ------------------------------------

@@ -3,14 +3,15 @@
 //
 // One force evaluation enqueues, on the context's stream:
 //   reset counters -> bounding box + root cube -> 63-bit keys -> radix sort
-//   (7 passes of 9-bit digits) -> gather the state into key order -> tree
-//   levels 0..20 -> leaf list -> upward moments -> grouped walk (+ closing
-//   kick)
-// then synchronises once and reads the device status word.  A node-pool or
-// walk-stack overflow is reported by the kernels (never silently dropped, as
-// the reference's GL path does at GpuBarnesHut.cpp:259-260 and :428), the
-// walk refuses to run on a truncated tree, and the host grows the pool and
-// re-runs the evaluation.
+//   (9-bit digits, as many as the tree is deep) -> gather the state into key
+//   order -> tree nodes and leaf list -> upward moments -> grouped walk ->
+//   evaluation of its lists (+ closing kick), or the per-particle walk
+// then synchronises once and reads the device status word.  A node-pool,
+// list-pool or walk-stack overflow is reported by the kernels (never silently
+// dropped, as the reference's GL path does at GpuBarnesHut.cpp:259-260 and
+// :428), no force is evaluated or kick given on a truncated tree or list, and
+// the host grows the pool and re-runs the evaluation.  The per-particle walk,
+// which gives its kicks as it goes, has no pool that could run out.
 #include "ngrav_gpu.h"
 
 #include "ctx_internal.cuh"

@@ -202,7 +202,7 @@ struct WalkParams {
     int smem_stack;                   // per-warp shared-memory walk stack: 1024, 2048 or 4096 entries
     int soft;                         // kSoftPlummer or kSoftSpline (softening.cuh)
     float ih;                         // spline: 1 / h (h = eps)
-    int p2p_tile;                     // sources per near batch of the evaluation (64, 128, 256; 0: its maximum)
+    int p2p_tile;                     // sources per near batch of the evaluation (64 or 128; 256 and 0: as many as fit)
     // learned opening test (walk_lmac_kernel)
     int learned;
     float lm_log2b;                   // log2 of the per-target error budget

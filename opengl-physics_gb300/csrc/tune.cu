@@ -130,7 +130,7 @@ int ngrav_gpu_autotune(ngrav_gpu_ctx* ctx, const ngrav_gpu_tune_opts* o, ngrav_g
     if (out) {
         std::memset(out, 0, sizeof(*out));
         out->leaf_capacity = best.ncrit;
-        out->p2p_tile = best.tile ? best.tile : 256;
+        out->p2p_tile = best.tile ? best.tile : 256;  // one and the same setting
         out->walk_stack = best.stack;
         out->ms_before = base.ms;
         out->ms_after = fin.ms;
