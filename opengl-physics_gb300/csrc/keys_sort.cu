@@ -651,9 +651,11 @@ __global__ void __launch_bounds__(THREADS, 1) rs_single_kernel(unsigned long lon
 }
 
 constexpr int kRsSingleMax = 1024 * kRsItems;
-// Tiles up to which a pass is two launches (FEW): the sort of 16,384 bodies (4
-// tiles) takes 78 us with three and 63 with two, of 131,071 (32 tiles) 82 and 97.
-constexpr int kRsFewTiles = 12;
+// Tiles up to which a pass is two launches (FEW).  Sort phase with three and with
+// two, Plummer sphere, 4 passes: 4 tiles 78 and 63 us, 12 78 and 64, 20 82 and 70,
+// 28 81 and 74, 32 83 and 98; galaxy, 5 passes: 96 and 78, 99 and 80, 101 and 85,
+// 101 and 91, 101 and 121.
+constexpr int kRsFewTiles = 28;
 
 constexpr int rs_single_smem(int threads) {
     return threads * kRsItems * (int)(sizeof(unsigned long long) + sizeof(unsigned));
