@@ -232,6 +232,12 @@ struct Forest {
     float4* frame = nullptr;          // per system: its key frame (kFrame)
 };
 
+// Packed FP32 pair arithmetic (two lanes of one register pair per op).
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
+
 // Error-free steps.  Every rounding is asked for by name: an operand may be a
 // product after inlining, and one fused into the sum, but not into its error,
 // would be counted twice.

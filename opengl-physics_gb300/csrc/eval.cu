@@ -53,6 +53,7 @@
 // SM, for L1 reuse: 1 to 3 % slower, most of shared memory being in use.
 #include "engine.cuh"
 #include "softening.cuh"
+#include "walk_common.cuh"
 
 namespace ngrav {
 
@@ -88,23 +89,6 @@ struct __align__(16) EvalSmem {
 };
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ int excl_scan(int v, int lane, int& total) {
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    total = __shfl_sync(0xffffffffu, x, 31);
-    return x - v;
-}
-
-// Packed FP32 pair arithmetic (two lanes of one register pair per op).
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
 
 // Two sources against target t: the reference's softened pair
 // (Solvers.cpp:19-38, AccumPairPlummer) for each, FP32.
@@ -543,7 +527,7 @@ __global__ void __launch_bounds__(kEvalThreads, kEvalMinBlocks) eval_kernel(Node
             }
             __syncwarp();
             int tot;
-            const int ex0 = excl_scan(cnt[0] + cnt[1], lane, tot), ex1 = ex0 + cnt[0];
+            const int ex0 = warp_excl_scan(cnt[0] + cnt[1], lane, tot), ex1 = ex0 + cnt[0];
             // whole windows, the wide ones if there is one, unless this is
             // the end of the list (or the batch does not fill one)
             const bool last = W.pos + kBatch >= nnear;

@@ -94,10 +94,10 @@ __device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf
 __device__ __forceinline__ float vsub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float vrsqrt(float a) { return rsqrtf(a); }
 __device__ __forceinline__ float vneg(float a) { return -a; }
-__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 vsub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return add2(a, b); }
+__device__ __forceinline__ float2 vmul(float2 a, float2 b) { return mul2(a, b); }
+__device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return fma2(a, b, c); }
+__device__ __forceinline__ float2 vsub(float2 a, float2 b) { return fma2(b, dup2(-1.f), a); }
 __device__ __forceinline__ float2 vrsqrt(float2 a) { return make_float2(rsqrtf(a.x), rsqrtf(a.y)); }
 __device__ __forceinline__ float2 vneg(float2 a) { return make_float2(-a.x, -a.y); }
 template <class V>

@@ -82,11 +82,6 @@ struct __align__(16) PpSmem {
     unsigned char bmask[64];
 };
 
-__device__ __forceinline__ float2 pp_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 pp_mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 pp_fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 pp_dup(float v) { return make_float2(v, v); }
-
 // Two sources or node centres (double-float) of one lane, and their members.
 struct PpPair {
     float2 x, y, z, m;
@@ -98,14 +93,14 @@ struct PpPair {
 template <bool SPLIT>
 __device__ __forceinline__ void pp_offset(const PpSmem& sm, int t, const PpPair& q, float2& dx, float2& dy, float2& dz) {
     const float4 h = sm.hi[t];
-    dx = pp_add(q.x, pp_dup(-h.x));
-    dy = pp_add(q.y, pp_dup(-h.y));
-    dz = pp_add(q.z, pp_dup(-h.z));
+    dx = add2(q.x, dup2(-h.x));
+    dy = add2(q.y, dup2(-h.y));
+    dz = add2(q.z, dup2(-h.z));
     if (SPLIT) {
         const float4 l = sm.lo[t];
-        dx = pp_add(dx, pp_add(q.lx, pp_dup(-l.x)));
-        dy = pp_add(dy, pp_add(q.ly, pp_dup(-l.y)));
-        dz = pp_add(dz, pp_add(q.lz, pp_dup(-l.z)));
+        dx = add2(dx, add2(q.lx, dup2(-l.x)));
+        dy = add2(dy, add2(q.ly, dup2(-l.y)));
+        dz = add2(dz, add2(q.lz, dup2(-l.z)));
     }
 }
 
@@ -171,19 +166,19 @@ struct PpWalk {
             const bool a = (m[0] >> t) & 1u, b = (m[1] >> t) & 1u;
             float2 dx, dy, dz;
             pp_offset<true>(sm, t, q, dx, dy, dz);
-            const float2 r2 = pp_fma(dx, dx, pp_fma(dy, dy, pp_mul(dz, dz)));
+            const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
             float2 f = make_float2(pair_factor<SOFT>(r2.x, q.m.x, wp.eps2, wp.ih),
                                    pair_factor<SOFT>(r2.y, q.m.y, wp.eps2, wp.ih));
-            float2 ir5 = pp_dup(0.f), qdx = ir5, qdy = ir5, qdz = ir5;
+            float2 ir5 = dup2(0.f), qdx = ir5, qdy = ir5, qdz = ir5;
             if (QUAD) {
-                qdx = pp_fma(qxx, dx, pp_fma(qxy, dy, pp_mul(qxz, dz)));
-                qdy = pp_fma(qxy, dx, pp_fma(qyy, dy, pp_mul(qyz, dz)));
-                qdz = pp_fma(qxz, dx, pp_fma(qyz, dy, pp_mul(qzz, dz)));
-                const float2 qd2 = pp_fma(dx, qdx, pp_fma(dy, qdy, pp_mul(dz, qdz)));
+                qdx = fma2(qxx, dx, fma2(qxy, dy, mul2(qxz, dz)));
+                qdy = fma2(qxy, dx, fma2(qyy, dy, mul2(qyz, dz)));
+                qdz = fma2(qxz, dx, fma2(qyz, dy, mul2(qzz, dz)));
+                const float2 qd2 = fma2(dx, qdx, fma2(dy, qdy, mul2(dz, qdz)));
                 const float2 ir = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-                const float2 ir2 = pp_mul(ir, ir);
-                ir5 = pp_mul(pp_mul(ir2, ir2), ir);
-                f = pp_fma(pp_mul(pp_dup(-2.5f), qd2), pp_mul(ir5, ir2), f);
+                const float2 ir2 = mul2(ir, ir);
+                ir5 = mul2(mul2(ir2, ir2), ir);
+                f = fma2(mul2(dup2(-2.5f), qd2), mul2(ir5, ir2), f);
                 ir5.x = a ? ir5.x : 0.f;
                 ir5.y = b ? ir5.y : 0.f;
             }
@@ -258,7 +253,7 @@ struct PpWalk {
                 if (t >= nt) break;
                 float2 dx, dy, dz;
                 pp_offset<SPLIT>(sm, t, q, dx, dy, dz);
-                const float2 r2 = pp_fma(dx, dx, pp_fma(dy, dy, pp_mul(dz, dz)));
+                const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
                 float2 f = make_float2(pair_factor<SOFT>(r2.x, q.m.x, wp.eps2, wp.ih),
                                        pair_factor<SOFT>(r2.y, q.m.y, wp.eps2, wp.ih));
                 f.x = (m[0] >> t) & 1u ? f.x : 0.f;
