@@ -43,8 +43,8 @@
 // and 3.6e-16 in another; FP64 terms 1.8e-16 and 5.7e-16.
 //
 // Measured (GB300, one diagnostics call on a Plummer sphere in tree order):
-// 131,071 particles 299 ms with FP64 terms -> 18.0 ms (0.69 of the FP32 pipe's
-// 54-operation time), 16,384 15.0 -> 0.37 ms, 2,048 (FP64 blocks of 32 sources
+// 131,071 particles 300 ms with FP64 terms -> 17.4 to 18.0 ms (the kernel 17.0: 0.68 of
+// the FP32 pipe's 54-operation time), 16,384 15.0 -> 0.37 ms, 2,048 (FP64 blocks of 32 sources
 // instead of whole rows) 1.87 -> 0.17 ms; spline, 20,011: 53.6 -> 0.7 ms.
 // Particles not yet in tree order have wide frames, so more pairs take
 // refine_pair: 45 ms at 131,071.
